@@ -276,9 +276,10 @@ static int load_matrix(Matrix& mx, const uint8_t* blob, size_t nbytes, const uin
 }
 
 static int finish_model(Model* M) {
-  size_t need = 0;
+  size_t need = 0, widest = 0;
   for (auto& m : M->mats) {
     if (m.fmt != kFmtNone && m.dev.group) {
+      widest = std::max(widest, static_cast<size_t>(m.K));
       need = std::max(need, gemv_partial_floats(m.dev, 8));
       if (m.K % 512 == 0) need = std::max(need, gemm_t5_plane_floats(m.dev, 64));   // planes of the tcgen05 path
     }
@@ -295,6 +296,9 @@ static int finish_model(Model* M) {
     const cudaError_t e2 = cudaMalloc(&M->d_row_scale, 4096 * sizeof(float));
     if (e2 != cudaSuccess) return cuda_fail("cudaMalloc (row factors)", e2);
     M->row_scale_floats = 4096;
+    const cudaError_t e3 = cudaMalloc(&M->d_x16, widest * 64 * sizeof(__half));   // the fused tensor-core path's rows
+    if (e3 != cudaSuccess) return cuda_fail("cudaMalloc (fp16 activations)", e3);
+    M->x16_halfs = widest * 64;
   }
   return kOk;
 }
@@ -363,24 +367,29 @@ static int grow(T** buf, size_t* have, size_t want, const char* what) {
   return kOk;
 }
 
+// Activations for the fp16 tensor-core paths: fp16 as they are, fp32 converted with a range factor per row.  *unscale =
+// the factors' inverses (null: none).
+static int half_rows(Model* M, const void* x, bool x_half, int m, int K, const __half** x16, const float** unscale, cudaStream_t st) {
+  *x16 = static_cast<const __half*>(x);
+  *unscale = nullptr;
+  if (x_half) return kOk;
+  int rc;
+  if ((rc = grow(&M->d_x16, &M->x16_halfs, static_cast<size_t>(m) * K, "cudaMalloc (fp16 activations)"))) return rc;
+  if ((rc = grow(&M->d_row_scale, &M->row_scale_floats, static_cast<size_t>(2) * m, "cudaMalloc (row factors)"))) return rc;
+  if ((rc = launch_rows_to_half(static_cast<const float*>(x), M->d_x16, m, K, M->d_row_scale, st))) return rc;
+  *x16 = M->d_x16;
+  *unscale = M->d_row_scale + m;
+  return kOk;
+}
+
 // Decode + GEMM (the reference's path for more than eight rows, kernels/llmrt.cu:1827-1841): tile rows are decoded to
 // fp16 weights in chunks that fit the scratch (grown on first use, at most kDecodeScratchBytes) and multiplied on the
 // tensor cores.
 constexpr size_t kDecodeScratchBytes = size_t(64) << 20;
 
-static int linear_decode_gemm(Model* M, Matrix& mx, const void* x, bool x_half, int m, float* y, int ldy,
+static int linear_decode_gemm(Model* M, Matrix& mx, const __half* x16, const float* unscale, int m, float* y, int ldy,
                               cudaStream_t st) {
   int rc;
-  const __half* x16 = static_cast<const __half*>(x);
-  const float* unscale = nullptr;
-  if (!x_half) {
-    if ((rc = grow(&M->d_x16, &M->x16_halfs, static_cast<size_t>(m) * mx.K, "cudaMalloc (fp16 activations)"))) return rc;
-    if ((rc = grow(&M->d_row_scale, &M->row_scale_floats, static_cast<size_t>(2) * m, "cudaMalloc (row factors)"))) return rc;
-    if ((rc = launch_row_scales(static_cast<const float*>(x), m, mx.K, M->d_row_scale, st))) return rc;
-    if ((rc = launch_to_half_rows(static_cast<const float*>(x), M->d_x16, m, mx.K, M->d_row_scale, st))) return rc;
-    x16 = M->d_x16;
-    unscale = M->d_row_scale + m;
-  }
   const int NT = mx.N / kTileRows;
   const size_t row_halfs = static_cast<size_t>(kTileRows) * mx.K;
   const int fit = static_cast<int>(std::max<size_t>(1, kDecodeScratchBytes / 2 / row_halfs));
@@ -392,8 +401,8 @@ static int linear_decode_gemm(Model* M, Matrix& mx, const void* x, bool x_half, 
     rc = reads_pairs(mx, 1) ? launch_decode_weights_rows(mx.pair, M->d_w16, tr0, tr1, st) : kErrTooLarge;   // two weights per lookup
     if (rc == kErrTooLarge) rc = launch_decode_weights_rows(mx.dev, M->d_w16, tr0, tr1, st);
     if (rc) return rc;
-    if ((rc = launch_gemm_tc(x16, M->d_w16, y + static_cast<size_t>(tr0) * kTileRows, m, (tr1 - tr0) * kTileRows, mx.K,
-                             ldy, M->d_partials, M->partial_floats, unscale, st)))
+    if ((rc = launch_gemm_w16(x16, M->d_w16, y + static_cast<size_t>(tr0) * kTileRows, m, (tr1 - tr0) * kTileRows, mx.K,
+                              ldy, M->d_partials, M->partial_floats, unscale, st)))
       return rc;
   }
   return kOk;
@@ -409,18 +418,20 @@ int linear_device(Model* M, Matrix& mx, const void* x, bool x_half, int m, float
   // path 0: up to eight rows the fused decode + product kernels; 9 .. 64 rows the decode + tcgen05 GEMM (decoded weights
   // go to tensor memory, never to DRAM); more rows, or shapes that kernel does not take, decode to fp16 weights in DRAM
   // and a tensor-core GEMM over them (the decode is paid once however many rows follow).  path 3 forces the tcgen05 kernel.
-  if (path == 3 || (path == 0 && m >= debug_knobs().t5_min_rows && m <= 64)) {
-    if (!x_half) {   // range factors of the rows, once for whichever layout takes the product
-      if (const int rc = grow(&M->d_row_scale, &M->row_scale_floats, 128, "cudaMalloc (row factors)")) return rc;
-      if (const int rc = launch_row_scales(static_cast<const float*>(x), m, mx.K, M->d_row_scale, st)) return rc;
-    }
+  const bool coded = path == 3 || (path == 0 && m >= debug_knobs().t5_min_rows && m <= 64);
+  const bool gemm = path == 2 || (path == 0 && m > 16);
+  const __half* x16 = nullptr;
+  const float* unscale = nullptr;
+  if (coded || gemm)
+    if (const int rc = half_rows(M, x, x_half, m, mx.K, &x16, &unscale, st)) return rc;
+  if (coded) {
     int rc = kErrTooLarge;
     if (reads_pairs(mx, 1))   // two weights per lookup; falls through where the larger units leave no room
-      rc = launch_gemm_coded(mx.pair, x, x_half, m, y, ldy, M->d_partials, M->partial_floats, M->d_row_scale, st);
-    if (rc == kErrTooLarge) rc = launch_gemm_coded(mx.dev, x, x_half, m, y, ldy, M->d_partials, M->partial_floats, M->d_row_scale, st);
+      rc = launch_gemm_coded(mx.pair, x16, unscale, m, y, ldy, M->d_partials, M->partial_floats, st);
+    if (rc == kErrTooLarge) rc = launch_gemm_coded(mx.dev, x16, unscale, m, y, ldy, M->d_partials, M->partial_floats, st);
     if (rc != kErrTooLarge || path == 3) return rc;
   }
-  if (path == 2 || (path == 0 && m > 16)) return linear_decode_gemm(M, mx, x, x_half, m, y, ldy, st);
+  if (gemm) return linear_decode_gemm(M, mx, x16, unscale, m, y, ldy, st);
   const size_t xe = x_half ? 2 : 4;
   for (int r0 = 0; r0 < m; r0 += 8) {
     const int mm = std::min(8, m - r0);

@@ -10,7 +10,7 @@
 //    so four consumer warps form a TEAM that decodes the same column segment of four consecutive tile rows: warp q
 //    fills lanes 32 q .. 32 q + 31.  A lane decodes two rows (l and l + 32 of its tile), hence two A tiles per step:
 //    tile "a" = rows l of the four tile rows, tile "b" = rows l + 32; they accumulate into two D tiles.
-//  * X is the B operand, converted once per block to fp16 in shared memory in the canonical K-major layout without
+//  * X is the B operand, placed once per block in shared memory in the canonical K-major layout without
 //    swizzle (8 x 16-byte core matrices; 128 bytes between K-adjacent core matrices, 8192 between 8-token groups) for
 //    the block's 512 weight columns.
 //  * D (fp32) lives in tensor memory, double-buffered: while the teams decode the next four tile rows, the previous
@@ -27,6 +27,7 @@
 #include <type_traits>
 
 #include "lw_ring.cuh"
+#include "lw_tcgen05.cuh"
 
 namespace lw {
 
@@ -41,74 +42,11 @@ constexpr uint32_t kT5TmemCols = 512;
 
 struct GemmT5Args {
   RingArgs r;          // r.nsets = K / 512 column sets; r.tr0 / r.ntr unused (all tile rows)
-  const void* x;       // activations [m][K], fp16 or fp32
+  const __half* x;     // activations [m][K]
   float* planes;       // P[K / 512][m][N]
-  const float* row_scale;   // fp32 x only (else null): factor per row that keeps it inside fp16's range
-  int x_is_half;
   int m;               // tokens (rows of x), 1 .. ntok
   int ntok;            // N of the MMA: m rounded up to a multiple of 16
 };
-
-// ------------------------------------------------------------------------------------------------ tcgen05 wrappers
-
-__device__ __forceinline__ void tmem_alloc(uint32_t* smem_dst, uint32_t cols) {
-  asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_addr(smem_dst)), "r"(cols)
-               : "memory");
-  asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
-}
-__device__ __forceinline__ void tmem_dealloc(uint32_t taddr, uint32_t cols) {
-  asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(taddr), "r"(cols) : "memory");
-}
-__device__ __forceinline__ void tc_fence_before() { asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory"); }
-__device__ __forceinline__ void tc_fence_after() { asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory"); }
-
-// 16 registers of this thread -> its tensor-memory lane, 16 consecutive columns from taddr
-__device__ __forceinline__ void tmem_store16(uint32_t taddr, const uint32_t (&v)[16]) {
-  asm volatile(
-      "tcgen05.st.sync.aligned.32x32b.x16.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15, %16};"
-      ::"r"(taddr), "r"(v[0]), "r"(v[1]), "r"(v[2]), "r"(v[3]), "r"(v[4]), "r"(v[5]), "r"(v[6]), "r"(v[7]), "r"(v[8]),
-      "r"(v[9]), "r"(v[10]), "r"(v[11]), "r"(v[12]), "r"(v[13]), "r"(v[14]), "r"(v[15])
-      : "memory");
-}
-__device__ __forceinline__ void tmem_wait_store() { asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory"); }
-__device__ __forceinline__ void tmem_load8(uint32_t taddr, uint32_t (&v)[8]) {
-  asm volatile("tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
-               : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]), "=r"(v[4]), "=r"(v[5]), "=r"(v[6]), "=r"(v[7])
-               : "r"(taddr)
-               : "memory");
-}
-__device__ __forceinline__ void tmem_wait_load() { asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory"); }
-
-// D[128 x N] (+)= A[128 x 16] (tensor memory) . B[N x 16]^T (shared memory descriptor), fp16 inputs, fp32 accumulate
-__device__ __forceinline__ void mma_ts_f16(uint32_t d_tmem, uint32_t a_tmem, uint64_t b_desc, uint32_t idesc, bool accumulate) {
-  const uint32_t acc = accumulate ? 1u : 0u;
-  asm volatile(
-      "{\n\t"
-      ".reg .pred p;\n\t"
-      "setp.ne.b32 p, %4, 0;\n\t"
-      "tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p;\n\t"
-      "}\n" ::"r"(d_tmem),
-      "r"(a_tmem), "l"(b_desc), "r"(idesc), "r"(acc)
-      : "memory");
-}
-// the barrier is arrived on once every MMA this thread has issued so far has completed
-__device__ __forceinline__ void mma_commit(uint64_t* bar) {
-  asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(smem_addr(bar)) : "memory");
-}
-__device__ __forceinline__ void mbar_arrive(uint64_t* bar) {
-  asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(smem_addr(bar)) : "memory");
-}
-
-// Shared-memory matrix descriptor of a K-major operand without swizzle: core matrices of 8 rows x 16 bytes,
-// `lbo` bytes between core matrices adjacent in K, `sbo` bytes between 8-row groups (all multiples of 16).
-__device__ __forceinline__ uint64_t smem_desc_kmajor(uint32_t saddr, uint32_t lbo, uint32_t sbo) {
-  return static_cast<uint64_t>((saddr >> 4) & 0x3FFFu) | (static_cast<uint64_t>((lbo >> 4) & 0x3FFFu) << 16) |
-         (static_cast<uint64_t>((sbo >> 4) & 0x3FFFu) << 32) | (1ull << 46);   // bit 46: descriptor version of this architecture
-}
-// Instruction descriptor: fp32 accumulator, fp16 A and B, both K-major, M = 128, N = n
-__host__ __device__ constexpr uint32_t idesc_f16_m128(int n) {
-  return (1u << 4) | (static_cast<uint32_t>(n >> 3) << 17) | (static_cast<uint32_t>(128 >> 4) << 24);
-}
 
 __device__ __forceinline__ uint32_t pack_half2(float lo, float hi) {
   const __half2 h = __halves2half2(__float2half_rn(lo), __float2half_rn(hi));
@@ -116,31 +54,6 @@ __device__ __forceinline__ uint32_t pack_half2(float lo, float hi) {
 }
 __device__ __forceinline__ float entry_value(uint32_t e, int which) {
   return static_cast<float>(static_cast<int>(static_cast<int8_t>((e >> (8 * which)) & 255u)));
-}
-
-// bounded waits that also end when another warp of the block has given up
-__device__ __forceinline__ bool t5_wait(uint64_t* bar, uint32_t parity, const RingArgs& A, volatile int* abort_flag) {
-  const uint32_t addr = smem_addr(bar);
-  for (uint32_t i = 0; i < A.wait_limit; ++i) {
-    uint32_t done;
-    asm volatile(
-        "{\n\t.reg .pred p;\n\t"
-        "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
-        "selp.u32 %0, 1, 0, p;\n\t}"
-        : "=r"(done)
-        : "r"(addr), "r"(parity)
-        : "memory");
-    if (done) return true;
-    if ((i & 63u) == 63u && *abort_flag) return false;
-  }
-  atomicOr(A.err, 1u);
-  *abort_flag = 1;
-  return false;
-}
-// the same for a whole warp: every lane gets the same answer, so that the warp stays converged for the .aligned
-// tensor-memory instructions that follow
-__device__ __forceinline__ bool t5_wait_warp(uint64_t* bar, uint32_t parity, const RingArgs& A, volatile int* abort_flag) {
-  return __all_sync(0xffffffffu, t5_wait(bar, parity, A, abort_flag));
 }
 
 // LOG_R: copies of the decode table in THIS kernel (8: half of what the chains' leading zero bits allow, because the
@@ -234,25 +147,17 @@ __global__ void __launch_bounds__(kT5Threads, 1) k_gemm_t5(const __grid_constant
     ring_produce(M, RA, RM, nmine, warp - kT5Consumers, lane);        // ---- producers: the staging ring
   }
 
-  // ---- X -> fp16 in the canonical K-major layout (all warps but the producers, which are already copying)
+  // ---- X in the canonical K-major layout (all warps but the producers, which are already copying)
   if (warp < kT5Consumers || warp == kT5Consumers + kT5Producers) {
     const int nthr = (kT5Consumers + 1) * 32;
     const int tid = warp < kT5Consumers ? threadIdx.x : kT5Consumers * 32 + lane;
-    // one thread converts eight consecutive K values of one token: one 16-byte row of a core matrix
+    // one thread places eight consecutive K values of one token: one 16-byte row of a core matrix
     for (int i = tid; i < ntok * (kT5SetK / 8); i += nthr) {
       const int n = i / (kT5SetK / 8), kc = i % (kT5SetK / 8);
       uint4 v = make_uint4(0u, 0u, 0u, 0u);
       if (n < A.m) {
         const size_t src = static_cast<size_t>(n) * M.K + static_cast<size_t>(set) * kT5SetK + kc * 8;
-        if (A.x_is_half) {
-          v = __ldg(reinterpret_cast<const uint4*>(static_cast<const __half*>(A.x) + src));
-        } else {
-          const float4 f0 = __ldg(reinterpret_cast<const float4*>(static_cast<const float*>(A.x) + src));
-          const float4 f1 = __ldg(reinterpret_cast<const float4*>(static_cast<const float*>(A.x) + src) + 1);
-          const float rs = A.row_scale ? A.row_scale[n] : 1.f;   // not __ldg: written by the kernel just before
-          v = make_uint4(pack_half2(f0.x * rs, f0.y * rs), pack_half2(f0.z * rs, f0.w * rs), pack_half2(f1.x * rs, f1.y * rs),
-                         pack_half2(f1.z * rs, f1.w * rs));
-        }
+        v = *reinterpret_cast<const uint4*>(A.x + src);
       }
       *reinterpret_cast<uint4*>(xs + (n >> 3) * (kT5SetK / 8 * 128) + kc * 128 + (n & 7) * 16) = v;
     }
@@ -271,7 +176,7 @@ __global__ void __launch_bounds__(kT5Threads, 1) k_gemm_t5(const __grid_constant
       bool ok = true;
       for (int it = 0; it < items && ok; ++it) {
         const int db = it & 1;
-        if (it >= 2) ok = t5_wait(d_empty + db, ((it >> 1) - 1) & 1, RA, abort_flag);   // the epilogue of item it - 2 is done
+        if (it >= 2) ok = t5_wait(d_empty + db, ((it >> 1) - 1) & 1, RA.wait_limit, RA.err, abort_flag);   // the epilogue of item it - 2 is done
         tc_fence_after();
         const uint32_t d_a = tmem + d_col0 + db * 2 * ntok, d_b = d_a + ntok;
         bool first = true;
@@ -280,7 +185,7 @@ __global__ void __launch_bounds__(kT5Threads, 1) k_gemm_t5(const __grid_constant
             for (int t = 0; t < kT5Teams && ok; ++t) {
               const int u = rd * kT5Teams + t;                        // the team-unit this team is on
               const uint32_t n = a_count[t]++, sl = n % kT5ASlots, ph = (n / kT5ASlots) & 1u;
-              ok = t5_wait(a_full + t * kT5ASlots + sl, ph, RA, abort_flag);
+              ok = t5_wait(a_full + t * kT5ASlots + sl, ph, RA.wait_limit, RA.err, abort_flag);
               if (!ok) break;
               tc_fence_after();
               const uint32_t koff = (u / SPLIT) * TW + (u % SPLIT) * KU + 16 * j;   // K offset inside the column set
@@ -305,7 +210,7 @@ __global__ void __launch_bounds__(kT5Threads, 1) k_gemm_t5(const __grid_constant
     // writes the plane of item `it` (tokens x 256 weight rows of its row group) from D buffer it % 2
     auto epilogue = [&](int it) {
       const int db = it & 1;
-      if (!t5_wait_warp(d_full + db, (it >> 1) & 1, RA, abort_flag)) return false;
+      if (!t5_wait_warp(d_full + db, (it >> 1) & 1, RA.wait_limit, RA.err, abort_flag)) return false;
       tc_fence_after();
       const int rg = bi + it * nb_set;
       float* plane = A.planes + static_cast<size_t>(set) * A.m * M.N;
@@ -404,7 +309,7 @@ __global__ void __launch_bounds__(kT5Threads, 1) k_gemm_t5(const __grid_constant
             // the team's next A slot, once the tensor core has read its previous contents
             const uint32_t sl = a_n % kT5ASlots, use = a_n / kT5ASlots;
             ++a_n;
-            if (use > 0 && !t5_wait_warp(a_empty + team * kT5ASlots + sl, (use - 1) & 1u, RA, abort_flag)) return false;
+            if (use > 0 && !t5_wait_warp(a_empty + team * kT5ASlots + sl, (use - 1) & 1u, RA.wait_limit, RA.err, abort_flag)) return false;
             tc_fence_after();
             tmem_store16(tmem + my_lanes + a_col0 + (team * kT5ASlots + sl) * 16, w);
             tmem_wait_store();

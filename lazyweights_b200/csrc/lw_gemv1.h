@@ -27,11 +27,9 @@ int launch_gemvm(const MatDev& M, const void* X, bool x_is_half, int m, float* p
 int launch_decode_codes_ring(const MatDev& M, uint8_t* out, bool expand, unsigned int* err, cudaStream_t st);
 
 // Decode + tcgen05 GEMM for up to 64 rows (lw_gemm_t5.cuh): planes[K / 512][m][N] of partial products, *terms = K / 512,
-// to be added by the caller; kErrTooLarge (nothing launched) where this kernel cannot take the product.  row_scale (may
-// be null): factor per row of X applied before the conversion to fp16; the caller multiplies the sums by the inverse.
+// to be added by the caller; kErrTooLarge (nothing launched) where this kernel cannot take the product.
 size_t gemm_t5_plane_floats(const MatDev& M, int m);
-int launch_gemm_t5(const MatDev& M, const void* X, bool x_is_half, const float* row_scale, int m, float* planes,
-                   unsigned int* err, cudaStream_t st, int* terms);
+int launch_gemm_t5(const MatDev& M, const __half* X, int m, float* planes, unsigned int* err, cudaStream_t st, int* terms);
 
 // fp16 weights of tile rows tr0 .. tr1 - 1 on the batch-1 kernel's decoder (lw_decw.cuh); kErrTooLarge (nothing
 // launched) where it cannot take the matrix.
@@ -51,6 +49,12 @@ DebugKnobs& debug_knobs();
 // Tensor map (a CUtensorMap, 128 bytes, 64-byte aligned) over an output buffer seen as bytes [rows][row_bytes] with boxes of
 // 64 rows x 32 bytes and the 32-byte swizzle; false where the driver does not offer the encoder or refuses the shape.
 bool make_row_tile_map(void* tensor_map, void* base, size_t row_bytes, size_t rows);
+// Tensor map over fp16 values [rows][K] with boxes of box_rows rows x 64 columns in the 128-byte swizzle: the operand slabs
+// of k_gemm_w16.
+bool make_half_slab_map(void* tensor_map, const void* base, size_t K, size_t rows, int box_rows);
+// Y = ordered sum over `terms` planes P[term][m][N] (k_sum_partials), times unscale per row if not null
+int launch_sum_partials(const float* P, float* Y, int m, int N, int ldy, int terms, const float* unscale, cudaStream_t st);
+unsigned int* error_word();   // device address of the error word on the current device
 // False with LW_TILE_OUT=0 in the environment (read once): the decode kernels then keep their 32-byte stores.
 bool tile_output_enabled();
 // Looks the tensor-map encoder up now (done when a matrix is loaded, so that a first decode inside a stream capture makes

@@ -169,9 +169,68 @@ __global__ void __launch_bounds__(kWarpsPerBlock * 32)
   }
 }
 
-}  // namespace lw
-#include "lw_gemm_tc.cuh"
-namespace lw {
+// fp32 activations enter the tensor cores as fp16, whose largest finite value is 65504: a row with larger entries (the
+// input of a down projection can be the product of two unnormalised projections) would turn into infinities and the
+// product into NaN.  Each row therefore gets a power-of-two factor that brings its largest |x| to at most 2^15 - exactly
+// 1 for every row that already fits, so ordinary inputs are converted bit for bit - and the product's rows are multiplied
+// by the inverse afterwards (exact: both are powers of two).
+//   dst[r][k] = half(src[r][k] * scales[r]); scales[r] = factor of row r, scales[m + r] = its inverse
+// One block per row; a thread holds up to 8 float4 of it between the maximum and the conversion (rows of up to 16384
+// values; the rest of a longer row is read again).  The row is one round trip to memory: 128 rows of 4096 values took 14 us
+// for the maxima and 4 us for the conversion as two kernels of scalar loads.
+constexpr int kToHalfThreads = 512, kToHalfHeld = 8;
+__global__ void __launch_bounds__(kToHalfThreads)
+    k_rows_to_half(const float* __restrict__ src, __half* __restrict__ dst, int K, int m, float* __restrict__ scales) {
+  __shared__ float part[kToHalfThreads / 32];
+  pdl_trigger();
+  pdl_wait();
+  const int r = blockIdx.x, quads = K / 4;
+  const float4* x = reinterpret_cast<const float4*>(src + static_cast<size_t>(r) * K);
+  uint2* out = reinterpret_cast<uint2*>(dst + static_cast<size_t>(r) * K);
+  const bool aligned = (reinterpret_cast<uintptr_t>(src) & 15u) == 0;   // the same for every row: K is a multiple of 256
+  auto load = [&](int k) {
+    if (aligned) return x[k];
+    const float* f = reinterpret_cast<const float*>(x) + 4 * k;
+    return make_float4(f[0], f[1], f[2], f[3]);
+  };
+  float4 v[kToHalfHeld];
+  float amax = 0.f;
+  auto largest = [&](const float4& a) { amax = fmaxf(fmaxf(amax, fmaxf(fabsf(a.x), fabsf(a.y))), fmaxf(fabsf(a.z), fabsf(a.w))); };
+#pragma unroll
+  for (int i = 0; i < kToHalfHeld; ++i) {
+    const int k = i * kToHalfThreads + threadIdx.x;
+    v[i] = k < quads ? load(k) : make_float4(0.f, 0.f, 0.f, 0.f);
+  }
+#pragma unroll
+  for (int i = 0; i < kToHalfHeld; ++i) largest(v[i]);
+  for (int k = kToHalfHeld * kToHalfThreads + threadIdx.x; k < quads; k += kToHalfThreads) largest(load(k));
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, o));
+  if ((threadIdx.x & 31) == 0) part[threadIdx.x >> 5] = amax;
+  __syncthreads();
+#pragma unroll
+  for (int w = 0; w < kToHalfThreads / 32; ++w) amax = fmaxf(amax, part[w]);
+  int e = 0;
+  if (amax > 32768.f && amax <= 3.0e38f) {   // frexp: amax = f 2^e with f in [0.5, 1)
+    frexpf(amax, &e);
+    e -= 15;
+  }
+  const float f = ldexpf(1.f, -e);
+  if (threadIdx.x == 0) {
+    scales[r] = f;
+    scales[m + r] = ldexpf(1.f, e);
+  }
+  auto halves = [&](const float4& a) {
+    const __half2 lo = __floats2half2_rn(a.x * f, a.y * f), hi = __floats2half2_rn(a.z * f, a.w * f);
+    return make_uint2(*reinterpret_cast<const uint32_t*>(&lo), *reinterpret_cast<const uint32_t*>(&hi));
+  };
+#pragma unroll
+  for (int i = 0; i < kToHalfHeld; ++i) {
+    const int k = i * kToHalfThreads + threadIdx.x;
+    if (k < quads) out[k] = halves(v[i]);
+  }
+  for (int k = kToHalfHeld * kToHalfThreads + threadIdx.x; k < quads; k += kToHalfThreads) out[k] = halves(load(k));
+}
 
 // Y[j, n] = sum over the `terms` partial rows of P[term, j, n], added in term order (no atomics: results do not
 // depend on scheduling).  One thread per four consecutive outputs: 16-byte loads, eight terms in flight.
@@ -268,6 +327,17 @@ bool make_row_tile_map(void* tensor_map, void* base, size_t row_bytes, size_t ro
                 CU_TENSOR_MAP_SWIZZLE_32B, CU_TENSOR_MAP_L2_PROMOTION_NONE, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
 }
 
+bool make_half_slab_map(void* tensor_map, const void* base, size_t K, size_t rows, int box_rows) {
+  const PFN_cuTensorMapEncodeTiled encode = tensor_map_encoder();
+  if (!encode || (reinterpret_cast<uintptr_t>(base) & 15u) || K % 64 || box_rows < 1 || box_rows > 256) return false;
+  const cuuint64_t dims[2] = {K, rows};
+  const cuuint64_t strides[1] = {K * 2};
+  const cuuint32_t box[2] = {64, static_cast<cuuint32_t>(box_rows)};
+  const cuuint32_t estr[2] = {1, 1};
+  return encode(static_cast<CUtensorMap*>(tensor_map), CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 2, const_cast<void*>(base), dims, strides, box, estr,
+                CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
+}
+
 // SMs of the current device (cached per device: a process may hold handles on several).
 int sm_count() {
   static std::atomic<int> per_device[64];
@@ -283,7 +353,7 @@ int sm_count() {
 }
 
 // Device address of the error word, for kernels of other translation units.
-static unsigned int* error_word() {
+unsigned int* error_word() {
   static std::mutex mu;
   static unsigned int* per_device[64] = {nullptr};
   int dev = 0;
@@ -412,6 +482,9 @@ int launch_gemv(const MatDev& M, const void* X, bool x_is_half, int m, float* Y,
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3((m * (M.N / 4) + 127) / 128);
     cfg.blockDim = dim3(128);
+    // more shared memory than the product kernel leaves free: blocks of the sum that move in beside it and wait there cost
+    // it 6 % (Q6_K 14336 x 4096, 8 rows: 52.5 instead of 49.6 us with the sum)
+    cfg.dynamicSmemBytes = 16 << 10;
     cfg.stream = st;
     cudaLaunchAttribute attr[1];
     attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
@@ -427,24 +500,15 @@ int launch_gemv(const MatDev& M, const void* X, bool x_is_half, int m, float* Y,
 }
 
 // Y[m, N] = X . W^T for up to 64 rows on the tcgen05 path: planes of partial products, then their ordered sum.
-// row_scale: the per-row range factors of fp32 activations and their inverses, 2 m floats filled by launch_row_scales
-// before this call; unused and may be null when X is fp16.
-int launch_gemm_coded(const MatDev& M, const void* X, bool x_is_half, int m, float* Y, int ldy, float* scratch,
-                      size_t scratch_floats, float* row_scale, cudaStream_t st) {
+int launch_gemm_coded(const MatDev& M, const __half* X, const float* unscale, int m, float* Y, int ldy, float* scratch,
+                      size_t scratch_floats, cudaStream_t st) {
   if (!gemv1_usable(M) || M.K % 512 || scratch_floats < gemm_t5_plane_floats(M, m)) {
     set_kernel_error_text("gemm (tcgen05)", "matrix not laid out for it, K not a multiple of 512, or scratch too small");
     return kErrTooLarge;
   }
-  if (!x_is_half && !row_scale) {
-    set_kernel_error_text("gemm (tcgen05)", "fp32 activations need scratch for their per-row factors");
-    return kErrArg;
-  }
   int terms = 0;
-  const int rc = launch_gemm_t5(M, X, x_is_half, x_is_half ? nullptr : row_scale, m, scratch, error_word(), st, &terms);
-  if (rc) return rc;
-  k_sum_partials<<<(m * (M.N / 4) + 127) / 128, 128, 0, st>>>(scratch, Y, m, M.N, ldy, terms,
-                                                             x_is_half ? nullptr : row_scale + m);
-  return check_launch("k_sum_partials");
+  const int rc = launch_gemm_t5(M, X, m, scratch, error_word(), st, &terms);
+  return rc ? rc : launch_sum_partials(scratch, Y, m, M.N, ldy, terms, unscale, st);
 }
 
 int launch_gemv_batch(int n, const MatDev* const* mats, const void* const* xs, bool x_is_half, float* const* ys,
@@ -552,37 +616,28 @@ extern "C" int lw_linear_static(void* handle, int id, const void* x_dev, int x_i
 
 namespace lw {
 
-int launch_row_scales(const float* X, int m, int K, float* scales, cudaStream_t st) {
-  k_row_scales<<<m, 256, 0, st>>>(X, K, m, scales);
-  return check_launch("k_row_scales");
+// A launch that may be set up while its predecessor in the stream still runs (see lw_device.cuh)
+template <typename... KArgs, typename... Args>
+static void launch_dependent(void (*kernel)(KArgs...), dim3 grid, dim3 block, cudaStream_t st, Args... args) {
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = grid;
+  cfg.blockDim = block;
+  cfg.stream = st;
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[0].val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = 1;
+  cudaLaunchKernelEx(&cfg, kernel, static_cast<KArgs>(args)...);
 }
 
-// dst = fp16 of src [m, K] with row r multiplied by scales[r] (launch_row_scales)
-int launch_to_half_rows(const float* src, __half* dst, int m, int K, const float* scales, cudaStream_t st) {
-  k_to_half_rows<<<dim3((K + 255) / 256, m), 256, 0, st>>>(src, dst, K, scales);
-  return check_launch("k_to_half_rows");
+int launch_rows_to_half(const float* src, __half* dst, int m, int K, float* scales, cudaStream_t st) {
+  launch_dependent(k_rows_to_half, dim3(m), dim3(kToHalfThreads), st, src, dst, K, m, scales);
+  return check_launch("k_rows_to_half");
 }
 
-// Y[m, rows] (row stride ldy, starting at column col0) = X[m, K] . W[rows, K]^T on the tensor cores
-// unscale (may be null): per-token factor applied to the finished products (inverse of the activations' range factors)
-int launch_gemm_tc(const __half* X, const __half* W, float* Y, int m, int rows, int K, int ldy, float* partials,
-                   size_t partial_capacity, const float* unscale, cudaStream_t st) {
-  if (m < 1 || rows % kGemmRows || K % kGemmK) {
-    set_kernel_error_text("gemm_tc", "shape must be a multiple of 64 rows x 64 columns");
-    return kErrArg;
-  }
-  // split K while the partial planes fit the scratch: one block per 64 rows streaming all of K leaves the SMs idle
-  int ks = 8;
-  while (ks > 1 && (K % (ks * kGemmK) || static_cast<size_t>(ks) * m * rows > partial_capacity || !partials)) ks /= 2;
-  dim3 grid(rows / kGemmRows, (m + kGemmTokens - 1) / kGemmTokens, ks);
-  if (ks == 1) {
-    k_gemm_tc<<<grid, 128, 0, st>>>(X, W, Y, m, K, ldy, K, 0, unscale);
-    return check_launch("k_gemm_tc");
-  }
-  k_gemm_tc<<<grid, 128, 0, st>>>(X, W, partials, m, K, rows, K / ks, static_cast<size_t>(m) * rows, nullptr);
-  int rc = check_launch("k_gemm_tc");
-  if (rc) return rc;
-  k_sum_partials<<<(m * (rows / 4) + 127) / 128, 128, 0, st>>>(partials, Y, m, rows, ldy, ks, unscale);
+int launch_sum_partials(const float* P, float* Y, int m, int N, int ldy, int terms, const float* unscale, cudaStream_t st) {
+  launch_dependent(k_sum_partials, dim3((m * (N / 4) + 127) / 128), dim3(128), st, P, Y, m, N, ldy, terms, unscale);
   return check_launch("k_sum_partials");
 }
 

@@ -1,0 +1,51 @@
+"""Products of several rows at the sizes where their kernels can go wrong: edges of the token tiles, row counts that are
+no multiple of the weight tiles, K that splits or does not, activations that need a range factor."""
+import numpy as np
+import pytest
+
+from oracle import lw_oracle as orc
+from tests import helpers
+
+pytestmark = pytest.mark.gpu
+# fp16 weights and activations: each factor of a term is off by at most 2^-11 of itself, so a sum of products of
+# independent signs is off by about 2^-11 sqrt(2) of its own size; 1e-3 of the largest result is the bar of every product.
+TOL = helpers.GEMV_TOL
+
+
+@pytest.fixture(scope="module")
+def lw():
+    helpers.build_library()
+    import torch
+    assert torch.cuda.is_available()
+    import lazyweights_b200 as pkg
+    yield pkg
+    assert pkg.lib().lw_kernel_error() == 0
+
+
+# N 64: half a weight tile; 192: one and a half; 320: two and a half; K 256: four slabs, no split; 14336: many
+@pytest.mark.parametrize("ty,n,k,rows", [("Q6_K", 64, 256, (65, 128)), ("Q4_K", 192, 512, (65, 80, 255, 256, 257)),
+                                         ("Q5_K", 320, 768, (17, 127, 129, 511, 512, 513)), ("IQ4_XS", 128, 14336, (66, 200)),
+                                         ("Q4_K", 4096, 2048, (300,))])
+@pytest.mark.parametrize("half", [True, False])
+def test_decode_and_gemm(lw, ty, n, k, rows, half):
+    import torch
+    q, side, sym, w, rng = helpers.seeded_case(ty, n, k, seed=n + k)
+    blob, _, _ = lw.bundle.encode_huf8(sym)
+    with lw.CodedMatrix(blob, n, sym.shape[1], ty, side) as mat:
+        for m in rows:
+            x = rng.standard_normal((m, k)).astype(np.float16 if half else np.float32)
+            if not half:
+                x[m // 2] *= 1e6   # beyond fp16: this row is scaled by a power of two on the way in and back on the way out
+            y = torch.full((m + 1, n), -7.0, device="cuda")
+            mat.linear("m", torch.from_numpy(x).cuda(), out=y[:m])
+            y = y.cpu().numpy()
+            assert (y[m] == -7.0).all()
+            ref = orc.gemv_f64(w, x.astype(np.float32))
+            for r in (0, m // 2, m - 1):
+                assert helpers.rel_err(y[r], ref[r]) <= TOL, (m, r)
+            rest = [r for r in range(m) if r != m // 2]
+            assert helpers.rel_err(y[rest], ref[rest]) <= TOL, m
+            if not half:   # 4-byte aligned activations
+                z = torch.empty(m * k + 1, device="cuda")
+                z[1:] = torch.from_numpy(x).cuda().reshape(-1)
+                assert torch.equal(mat.linear("m", z[1:].reshape(m, k)), torch.from_numpy(y[:m]).cuda())
