@@ -49,6 +49,7 @@ struct HostImage {
   std::vector<uint32_t> fat, symtab, cmp, group_base, words;
   std::vector<uint8_t> unit_slow;
   int KT = 0, T = 0, split = 1, pad = 0, max_len = 0, group = 0, index_bits = 0;
+  bool short_code = false;   // words of at most nine bits: read with the 512-window table, no unit classes
   double slow_fraction = 0.0;
   uint32_t max_unit = 0, max_tile = 0;
 };
@@ -63,10 +64,13 @@ static int check_side(const Matrix& mx, const uint8_t* side, size_t side_nbytes)
   return kOk;
 }
 
-// Matrices with a block format whose bundle code uses 11-bit words are re-coded at load with the same rule limited to
-// 10 bits (LW_RECODE=0, read at every load: keep the bundle's own code).  The symbols are the same; the device then holds
-// a code whose 1024-window table fits sixteen times where the 2048-window table fits eight times, and shared-memory
-// bank conflicts are what bounds the product kernels (Q4_K 4096 x 4096: 4.5 instead of 5.1 us per product).
+// Matrices with a block format whose bundle code has words of more than nine bits are re-coded at load with the same rule
+// limited to nine (LW_RECODE=0, read at every load: keep the bundle's own code).  The symbols are the same; the device
+// then holds a code whose 512-window table fits shared memory 32 times, once per lane, and whose groups of four symbols
+// need no refill check - shared-memory wavefronts and instructions are what bounds the kernels, not DRAM, which reads
+// 5 % more (paired 4-bit codes: 6.44 instead of 6.12 bits per pair).  Ten bits (16 copies) is where the first step of
+// this went; eight would leave 256 paired symbols no shorter words at all.
+constexpr int kRecodeBits = 9;
 static bool recode_wanted() {
   const char* e = getenv("LW_RECODE");
   return !(e && e[0] == '0');
@@ -80,11 +84,11 @@ static int prepare_matrix(const Matrix& mx, const uint8_t* blob, size_t nbytes, 
   if ((rc = check_side(mx, side, side_nbytes))) return rc;
   auto tab = std::make_unique<HuffTable>();
   if ((rc = table_from_lut(v.lut(), *tab))) return rc;
-  if (may_recode && recode_wanted() && mx.fmt != kFmtNone && tab->max_len > 10) {
+  if (may_recode && recode_wanted() && mx.fmt != kFmtNone && tab->max_len > kRecodeBits) {
     // validate and decode the bundle's blob, encode the symbols again with the shorter limit, lay that blob out
     std::vector<uint8_t> symbols(static_cast<size_t>(mx.N) * mx.Ks), shorter;
     if ((rc = walk_blob(v, *tab, default_split(mx.fmt), threads, nullptr, nullptr, symbols.data(), nullptr))) return rc;
-    rc = encode_huf8(symbols.data(), mx.N, mx.Ks, shorter, nullptr, 10, threads);
+    rc = encode_huf8(symbols.data(), mx.N, mx.Ks, shorter, nullptr, kRecodeBits, threads);
     symbols = std::vector<uint8_t>();
     if (rc == kOk) return prepare_matrix(mx, shorter.data(), shorter.size(), side, side_nbytes, threads, im, false);
     if (rc != kErrTooLarge) return rc;   // a payload at the format's 2^32-bit limit: the bundle's own code stays
@@ -145,6 +149,8 @@ static int prepare_matrix(const Matrix& mx, const uint8_t* blob, size_t nbytes, 
         }
       }
     }
+    im.short_code = group && tab->max_len <= kRecodeBits && !eg && !ei;
+    if (im.short_code) im.slow_fraction = 0.0;
     if (group) {
       const uint8_t gbit = static_cast<uint8_t>(1u << (group - kScanMinG));
       im.unit_slow.resize(scan.mask.size());
@@ -253,8 +259,8 @@ static int upload_matrix(Matrix& mx, const HostImage& im, const uint8_t* side, s
   tile_output_warm();
   mx.dev.side = side_nbytes ? d + off_side : nullptr;
   mx.dev.unit_slow = im.unit_slow.empty() ? nullptr : d + off_slow;
-  mx.dev.group = im.unit_slow.empty() ? 0 : im.group;
-  mx.dev.index_bits = im.index_bits;
+  mx.dev.group = im.unit_slow.empty() ? 0 : im.group;   // of a refill group; the 512-window readers take fours
+  mx.dev.index_bits = im.short_code ? 9 : im.index_bits;
   mx.dev.N = mx.N;
   mx.dev.K = mx.K;
   mx.dev.Ks = mx.Ks;

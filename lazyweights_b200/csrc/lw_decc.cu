@@ -25,7 +25,7 @@ static int launch_o(const MatDev& M, uint8_t* out, const CUtensorMap& tm, int tr
     const int rc = launch_o<FMT, G, IDXBITS, EXPAND, TILE_OUT>(M, out, tm, tr0, mid, err, st);
     return rc ? rc : launch_o<FMT, G, IDXBITS, EXPAND, TILE_OUT>(M, out, tm, mid, tr1, err, st);
   }
-  const size_t fixed = (size_t(1) << (M.index_bits + ring_log_copies(M.index_bits) + 2)) + kLutSize * 4 + ring_fixed_bytes(max_units) + kRingSlackWords * 4;
+  const size_t fixed = (size_t(1) << (M.index_bits + ring_log_copies(M.index_bits) + 2)) + (one_class(FMT, IDXBITS) ? 0 : kLutSize * 4) + ring_fixed_bytes(max_units) + kRingSlackWords * 4;
   const size_t buf_bytes = static_cast<size_t>(buf_words) * 4;
   if (fixed + buf_bytes > kSmemLimit) return kErrTooLarge;
   // with TILE_OUT every consumer warp also has a 2 KB area for its rows' bytes: about three consumers per four buffers
@@ -100,6 +100,7 @@ static int launch_i(const MatDev& M, uint8_t* out, bool expand, unsigned int* er
 
 template <int FMT>
 static int launch_bundle_code(const MatDev& M, uint8_t* out, bool expand, unsigned int* err, cudaStream_t st) {
+  if (M.index_bits == 9) return launch_e<FMT, 4, 9>(M, out, expand, err, st);
   switch (M.group) {
     case 3: return launch_x<FMT, 3>(M, out, expand, err, st);
     case 4: return launch_x<FMT, 4>(M, out, expand, err, st);

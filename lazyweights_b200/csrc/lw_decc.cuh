@@ -42,13 +42,14 @@ __global__ void __launch_bounds__(1024, 1) k_decode_codes_ring(const __grid_cons
   constexpr bool PAIR_LAYOUT = is_pair_layout(FMT);
   static_assert(!PAIR_LAYOUT || EXPAND, "a pair layout is written expanded");
   constexpr int NIDX = 1 << IDXBITS, R = 1 << LOG_R;
-  constexpr bool SINGLE = NIDX <= kLutSize;
+  constexpr bool ONE_CLASS = one_class(FMT, IDXBITS);
+  constexpr bool SINGLE = !ONE_CLASS;   // a single-copy table of all 2048 windows
   constexpr uint32_t MASK = static_cast<uint32_t>(NIDX - 1) << (LOG_R + 2);
   constexpr int kReplicatedTableBytes = NIDX * R * 4;
   extern __shared__ __align__(1024) uint8_t smem[];
   uint32_t* tab = reinterpret_cast<uint32_t*>(smem);
   uint32_t* tab1 = reinterpret_cast<uint32_t*>(smem + kReplicatedTableBytes);
-  uint8_t* stage0 = reinterpret_cast<uint8_t*>(tab1 + kLutSize);   // [warps][2 KB] when TILE_OUT; 1024-byte aligned
+  uint8_t* stage0 = reinterpret_cast<uint8_t*>(tab1 + (SINGLE ? kLutSize : 0));   // [warps][2 KB] when TILE_OUT; 1024-byte aligned
   RingMem RM;
   RM.carve(stage0 + (TILE_OUT ? RA.warps * WarpTileStage::kBytes : 0), RA);
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -124,7 +125,7 @@ __global__ void __launch_bounds__(1024, 1) k_decode_codes_ring(const __grid_cons
     uint8_t* oa = A.out + (static_cast<size_t>(u.tr) * kTileRows + lane) * A.row_bytes +
                   (static_cast<size_t>(u.j) * kTileSyms + u.seg * USYM) * OUT_PER_SYM;
     uint8_t* ob = oa + static_cast<size_t>(32) * A.row_bytes;
-    if (PAIR_LAYOUT || u.cls == 0) {   // a pair layout has no other class
+    if (ONE_CLASS || u.cls == 0) {
 #pragma unroll
       for (int c0 = 0; c0 < USYM; c0 += PER) {
         BytePack pa, pb;
@@ -145,7 +146,7 @@ __global__ void __launch_bounds__(1024, 1) k_decode_codes_ring(const __grid_cons
         }
         out32(u, c0 / PER, pa, pb, oa, ob);
       }
-    } else if constexpr (!PAIR_LAYOUT) {
+    } else if constexpr (!ONE_CLASS) {
 #pragma unroll 1
       for (int c0 = 0; c0 < USYM; c0 += PER) {
         BytePack pa, pb;

@@ -25,7 +25,7 @@ static int launch_o(const MatDev& M, __half* out, int tr0, int tr1, unsigned int
     const int rc = launch_o<FMT, G, IDXBITS, TILE_OUT>(M, out, tr0, mid, err, st);
     return rc ? rc : launch_o<FMT, G, IDXBITS, TILE_OUT>(M, out + static_cast<size_t>(mid - tr0) * kTileRows * M.K, mid, tr1, err, st);
   }
-  const size_t fixed = (size_t(1) << (M.index_bits + ring_log_copies(M.index_bits) + 2)) + kLutSize * 4 + 2 * kGemv1MaxSlots * 8 +
+  const size_t fixed = (size_t(1) << (M.index_bits + ring_log_copies(M.index_bits) + 2)) + (one_class(FMT, IDXBITS) ? 0 : kLutSize * 4) + 2 * kGemv1MaxSlots * 8 +
                        kGemv1MaxSlots * 4 + 16 + max_units * sizeof(UnitMeta) + kRingSlackWords * 4;
   const size_t buf_bytes = static_cast<size_t>(buf_words) * 4;
   if (fixed + buf_bytes > kSmemLimit) return kErrTooLarge;
@@ -91,6 +91,7 @@ static int launch_i(const MatDev& M, __half* out, int tr0, int tr1, unsigned int
 
 template <int FMT>
 static int launch_bundle_code(const MatDev& M, __half* out, int tr0, int tr1, unsigned int* err, cudaStream_t st) {
+  if (M.index_bits == 9) return launch_t<FMT, 4, 9>(M, out, tr0, tr1, err, st);
   switch (M.group) {
     case 3: return launch_x<FMT, 3>(M, out, tr0, tr1, err, st);
     case 4: return launch_x<FMT, 4>(M, out, tr0, tr1, err, st);

@@ -48,13 +48,14 @@ __global__ void __launch_bounds__(1024, 1) k_decw(const __grid_constant__ MatDev
   constexpr int NSU = TW / GW / SPLIT;   // sub-blocks per unit: four, or eight 16-weight ones of a Q6_K pair layout
   constexpr bool PAIR_LAYOUT = is_pair_layout(FMT);
   constexpr int NIDX = 1 << IDXBITS, R = 1 << LOG_R;
-  constexpr bool SINGLE = NIDX <= kLutSize;
+  constexpr bool ONE_CLASS = one_class(FMT, IDXBITS);
+  constexpr bool SINGLE = !ONE_CLASS;   // a single-copy table of all 2048 windows
   constexpr uint32_t MASK = static_cast<uint32_t>(NIDX - 1) << (LOG_R + 2);
   constexpr int kReplicatedTableBytes = NIDX * R * 4;
   extern __shared__ __align__(1024) uint8_t smem[];
   uint32_t* tab = reinterpret_cast<uint32_t*>(smem);
   uint32_t* tab1 = reinterpret_cast<uint32_t*>(smem + kReplicatedTableBytes);
-  uint8_t* stage0 = reinterpret_cast<uint8_t*>(tab1 + kLutSize);   // [warps][2 KB] when TILE_OUT; 1024-byte aligned
+  uint8_t* stage0 = reinterpret_cast<uint8_t*>(tab1 + (SINGLE ? kLutSize : 0));   // [warps][2 KB] when TILE_OUT; 1024-byte aligned
   RingMem RM;
   RM.carve(stage0 + (TILE_OUT ? RA.warps * WarpTileStage::kBytes : 0), RA);
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -140,7 +141,7 @@ __global__ void __launch_bounds__(1024, 1) k_decw(const __grid_constant__ MatDev
         }
       }
     };
-    if (PAIR_LAYOUT || cls == 0) {   // a pair layout has no other class
+    if (ONE_CLASS || cls == 0) {
       // the common class: groups of G symbols per refill check, everything unrolled (the phase of the groups is static)
 #pragma unroll
       for (int jj = 0; jj < NSU; ++jj) {
@@ -167,7 +168,7 @@ __global__ void __launch_bounds__(1024, 1) k_decw(const __grid_constant__ MatDev
           out16(jj * GW + (PAIR ? 2 * c0 : c0), pa, pb);
         }
       }
-    } else if constexpr (!PAIR_LAYOUT) {
+    } else if constexpr (!ONE_CLASS) {
       // the fallback classes, rolled up: window normalised per symbol (exact for any data), or the single-copy table
 #pragma unroll 1
       for (int jj = 0; jj < 4; ++jj) {

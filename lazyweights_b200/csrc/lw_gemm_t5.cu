@@ -9,8 +9,8 @@ namespace lw {
 
 constexpr size_t kSmemLimit = 227 * 1024;
 constexpr int kRingSlackWords = 96;
-// 8 copies of the decode table: 32 KB (1024 windows) or 64 KB (2048); 4 copies of a pair layout's 4096 windows
-constexpr int t5_log_copies(int index_bits) { return index_bits == 12 ? 2 : 3; }
+// Copies of the decode table: 16 of 512 windows or 8 of 1024 (32 KB), 8 of 2048 or 4 of a pair layout's 4096 (64 KB)
+constexpr int t5_log_copies(int index_bits) { return index_bits == 12 ? 2 : index_bits == 9 ? 4 : 3; }
 constexpr int kT5MinSlots = 17;   // sixteen consumer warps hold a unit each; the rest is run-ahead of the copies
 
 struct T5Plan {
@@ -38,7 +38,7 @@ static bool plan_t5(const MatDev& M, int m, T5Plan& p) {
     return false;
   }
   p.buf_words = (M.max_unit_words + 31u) & ~31u;
-  const size_t fixed = (size_t(1) << (M.index_bits + t5_log_copies(M.index_bits) + 2)) + (M.index_bits < kMaxLen ? kLutSize * 4 : 0) +
+  const size_t fixed = (size_t(1) << (M.index_bits + t5_log_copies(M.index_bits) + 2)) + (M.index_bits < kMaxLen && !one_class(FMT, M.index_bits) ? kLutSize * 4 : 0) +
                        static_cast<size_t>(p.ntok) * kT5SetK * 2 +
                        (2 * kT5Teams * kT5ASlots + 4) * 8 + 16 + ring_fixed_bytes(p.max_units) + kRingSlackWords * 4;
   if (fixed + static_cast<size_t>(p.buf_words) * 4 * kT5MinSlots > kSmemLimit) {
@@ -114,6 +114,7 @@ static int launch_g(const MatDev& M, const __half* X, int m, float* planes, unsi
 template <int FMT>
 static int launch_bundle_code(const MatDev& M, const __half* X, int m, float* planes, unsigned int* err,
                               cudaStream_t st, int* terms) {
+  if (M.index_bits == 9) return launch_t<FMT, 4, 9>(M, X, m, planes, err, st, terms);
   switch (M.group) {
     case 3: return launch_i<FMT, 3>(M, X, m, planes, err, st, terms);
     case 4: return launch_i<FMT, 4>(M, X, m, planes, err, st, terms);

@@ -56,6 +56,12 @@ __device__ __forceinline__ float entry_value(uint32_t e, int which) {
   return static_cast<float>(static_cast<int>(static_cast<int8_t>((e >> (8 * which)) & 255u)));
 }
 
+// a dependent call: readers without unit classes have no symbol-by-symbol form
+template <class TAG, class CH>
+__device__ __forceinline__ uint32_t slow_symbol(TAG, CH& ch, const uint32_t* tab1, uint32_t pad) {
+  return ch.slow_sym(tab1, pad);
+}
+
 // LOG_R: copies of the decode table in THIS kernel (8: half of what the chains' leading zero bits allow, because the
 // activations need the shared memory; lw::kRingLogCopies - LOG_R = the extra shift of every lookup).
 template <int FMT, int G, int IDXBITS, int LOG_R>
@@ -78,7 +84,8 @@ __global__ void __launch_bounds__(kT5Threads, 1) k_gemm_t5(const __grid_constant
   uint32_t* tab = reinterpret_cast<uint32_t*>(smem);
   // the single-copy table serves the units that hold an 11-bit code under a 1024-window table; with 2048 windows
   // replicated there are no such units and no such table
-  constexpr bool SINGLE = IDXBITS < kMaxLen;
+  constexpr bool ONE_CLASS = one_class(FMT, IDXBITS);
+  constexpr bool SINGLE = IDXBITS < kMaxLen && !ONE_CLASS;
   uint32_t* tab1 = reinterpret_cast<uint32_t*>(smem + kReplicatedTableBytes);       // [2048] single copy (if SINGLE)
   uint8_t* xs = reinterpret_cast<uint8_t*>(tab1 + (SINGLE ? kLutSize : 0));        // B operand: [ntok][512] fp16, canonical
   const int ntok = A.ntok;
@@ -287,9 +294,9 @@ __global__ void __launch_bounds__(kT5Threads, 1) k_gemm_t5(const __grid_constant
                 eb = cb.template sym<MASK>(smem, lane_off);
                 ca.end();
                 cb.end();
-              } else {
-                ea = ca.slow_sym(tab1, LOG_R + 2);
-                eb = cb.slow_sym(tab1, LOG_R + 2);
+              } else if constexpr (CLS == 2) {
+                ea = slow_symbol(cls_tag, ca, tab1, LOG_R + 2);
+                eb = slow_symbol(cls_tag, cb, tab1, LOG_R + 2);
               }
               if (PAIR) {
                 w[c] = pack_half2(__fsub_rn(__fmul_rn(s_a, entry_value(ea, 0)), o_a), __fsub_rn(__fmul_rn(s_a, entry_value(ea, 1)), o_a));
@@ -319,7 +326,8 @@ __global__ void __launch_bounds__(kT5Threads, 1) k_gemm_t5(const __grid_constant
           }
           return true;
         };
-        if (is_pair_layout(FMT) || cls == 0) ok = run_unit(std::integral_constant<int, 0>{});   // a pair layout has no other class
+        if (ONE_CLASS || cls == 0) ok = run_unit(std::integral_constant<int, 0>{});
+        else if constexpr (ONE_CLASS) ok = false;   // never reached
         else if (cls == 1 || !SINGLE) ok = run_unit(std::integral_constant<int, 1>{});
         else ok = run_unit(std::integral_constant<int, 2>{});
         if (!ok) break;

@@ -61,7 +61,7 @@ static bool plan_gemv1(const MatDev& M, int ntr, Gemv1Plan& p, int index_bits, i
   // LW_GEMV1_RING=16 where 36 staging buffers still fit (measured: no difference on the bench matrix).
   size_t fixed = 0;
   for (p.tile_ring_log2 = gemv1_env().ring >= 16 ? 4 : 3; p.tile_ring_log2 >= 3; --p.tile_ring_log2) {
-    fixed = (size_t(1) << (index_bits + log_copies + 2)) + kLutSize * 4 +
+    fixed = (size_t(1) << (index_bits + log_copies + 2)) + (one_class(FMT, index_bits) ? 0 : kLutSize * 4) +
             static_cast<size_t>(p.cols_per_set) * (kTileSyms + (has_offset ? 2 : 1) * (TW / sub_width(FMT))) * 4 +
             2 * kGemv1MaxSlots * 8 + kGemv1MaxSlots * 4 + 16 + (size_t(1) << p.tile_ring_log2) * (8 + SPLIT * kTileRows * 4) +
             p.max_units * sizeof(UnitMeta) + kRingSlackWords * 4;
@@ -186,6 +186,7 @@ static int launch_batch_g(int n, const MatDev* const* mats, const void* const* x
       if (mats[0]->index_bits == 12) return launch_batch_t<FMT, 3, 12>(n, mats, xs, x_is_half, partials, ys, err, st);
     return launch_batch_t<FMT, 3, 11>(n, mats, xs, x_is_half, partials, ys, err, st);
   } else {
+    if (mats[0]->index_bits == 9) return launch_batch_t<FMT, 4, 9>(n, mats, xs, x_is_half, partials, ys, err, st);
     switch (mats[0]->group) {
       case 3: return launch_batch_i<FMT, 3>(n, mats, xs, x_is_half, partials, ys, err, st);
       case 4: return launch_batch_i<FMT, 4>(n, mats, xs, x_is_half, partials, ys, err, st);
@@ -268,14 +269,18 @@ static int launch_t(const MatDev& M, const void* X, bool x_is_half, float* P, fl
   return kOk;
 }
 
-template <int FMT, int G>
-static int launch_i(const MatDev& M, const void* X, bool x_is_half, float* P, float* Y, unsigned int* err, cudaStream_t st) {
-  // LW_GEMV1_LOOKUP=limit: the comparator decoder instead of the table (a measurement switch, read once)
-  static const bool use_limit = [] {
+// LW_GEMV1_LOOKUP=limit: the comparator decoder instead of the table (a measurement switch, read once)
+static bool limit_reader_wanted() {
+  static const bool wanted = [] {
     const char* e = getenv("LW_GEMV1_LOOKUP");
     return e && std::string(e) == "limit";
   }();
-  if (use_limit && M.cmp_tab) return launch_t<FMT, G, 10, kGemv1LogCopies, kReaderLimit>(M, X, x_is_half, P, Y, err, st);
+  return wanted;
+}
+
+template <int FMT, int G>
+static int launch_i(const MatDev& M, const void* X, bool x_is_half, float* P, float* Y, unsigned int* err, cudaStream_t st) {
+  if (limit_reader_wanted() && M.cmp_tab) return launch_t<FMT, G, 10, kGemv1LogCopies, kReaderLimit>(M, X, x_is_half, P, Y, err, st);
   if (M.index_bits == 10) return launch_t<FMT, G, 10, kGemv1LogCopies>(M, X, x_is_half, P, Y, err, st);
   return launch_t<FMT, G, 11, ring_log_copies(11)>(M, X, x_is_half, P, Y, err, st);
 }
@@ -288,6 +293,7 @@ static int launch_g(const MatDev& M, const void* X, bool x_is_half, float* P, fl
     return launch_t<FMT, 3, 11, ring_log_copies(11)>(M, X, x_is_half, P, Y, err, st);
   } else {
     if (M.reader == 1) return launch_t<FMT, 3, 10, kGemv1LogCopies, kReaderFixed>(M, X, x_is_half, P, Y, err, st);
+    if (M.index_bits == 9 && !limit_reader_wanted()) return launch_t<FMT, 4, 9, ring_log_copies(9)>(M, X, x_is_half, P, Y, err, st);
     switch (M.group) {
       case 3: return launch_i<FMT, 3>(M, X, x_is_half, P, Y, err, st);
       case 4: return launch_i<FMT, 4>(M, X, x_is_half, P, Y, err, st);
@@ -309,7 +315,7 @@ bool gemv1_usable(const MatDev& M) {
            M.group == 3 && M.reader == 0;
   const bool fmt_ok = M.fmt >= kFmtQ4K && M.fmt <= kFmtIQ4XS;
   const int gmax = is_paired(M.fmt) ? 4 : 6;
-  return fmt_ok && (M.index_bits == 10 || M.index_bits == 11) && M.pad == kRingLogCopies + 2 && M.split == default_split(M.fmt) && M.unit_slow && M.row_done && M.group >= 3 &&
+  return fmt_ok && (M.index_bits == 9 || M.index_bits == 10 || M.index_bits == 11) && M.pad == kRingLogCopies + 2 && M.split == default_split(M.fmt) && M.unit_slow && M.row_done && M.group >= 3 &&
          M.group <= gmax;
 }
 

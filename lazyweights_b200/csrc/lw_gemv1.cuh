@@ -248,7 +248,8 @@ __device__ __forceinline__ void gemv1_block(const MatDev& M, const Gemv1Args& A,
   static_assert(!PAIR_LAYOUT || READER == kReaderTable, "pair layouts are read through their table");
   constexpr bool HAS_OFFSET = FMT == kFmtQ4K || FMT == kFmtQ5K || FMT == kFmtQ5KP;
   constexpr int NIDX = 1 << IDXBITS, R = 1 << LOG_R;              // windows, copies of the table
-  constexpr bool SINGLE = NIDX <= kLutSize;                       // a single-copy table of all 2048 windows beside it
+  constexpr bool ONE_CLASS = one_class(FMT, IDXBITS);
+  constexpr bool SINGLE = !ONE_CLASS;                             // a single-copy table of all 2048 windows beside it
   constexpr uint32_t MASK = static_cast<uint32_t>(NIDX - 1) << (LOG_R + 2);
   // the table area: the replicated Huffman table; or, for the other readers, [256][32] grid values (+ [12][32] offsets)
   constexpr int kReplicatedTableBytes = READER == kReaderTable ? NIDX * R * 4 : NIDX * R * 4 >= 34 * 1024 ? NIDX * R * 4 : 34 * 1024;
@@ -256,7 +257,7 @@ __device__ __forceinline__ void gemv1_block(const MatDev& M, const Gemv1Args& A,
   const RingArgs& RA = A.r;
   uint32_t* tab = reinterpret_cast<uint32_t*>(smem);
   uint32_t* tab1 = reinterpret_cast<uint32_t*>(smem + kReplicatedTableBytes);  // [2048] single copy
-  uint32_t* xq = tab1 + kLutSize;                                             // [cols_per_set][kTileSyms] words
+  uint32_t* xq = tab1 + (SINGLE ? kLutSize : 0);                                             // [cols_per_set][kTileSyms] words
   float* xscale = reinterpret_cast<float*>(xq + static_cast<size_t>(RA.cols_per_set) * kTileSyms);  // [cols][TW / GW]
   float* xg = xscale + static_cast<size_t>(RA.cols_per_set) * (TW / GW);      // [cols][TW / GW] sums (offset formats)
   const int ring = 1 << A.tile_ring_log2;
@@ -311,7 +312,7 @@ __device__ __forceinline__ void gemv1_block(const MatDev& M, const Gemv1Args& A,
 #pragma unroll
       for (int i = 0; i < T1_PRE; ++i) {   // windows beyond the replicated table (single-copy table only)
         const int idx = NIDX + i * nthr + static_cast<int>(threadIdx.x);
-        t1_pre[i] = idx < kLutSize ? __ldg(M.tab32 + idx) : 0u;
+        t1_pre[i] = SINGLE && idx < kLutSize ? __ldg(M.tab32 + idx) : 0u;
       }
     }
     if (!A.pdl) load_x(0);
@@ -343,9 +344,9 @@ __device__ __forceinline__ void gemv1_block(const MatDev& M, const Gemv1Args& A,
 #pragma unroll
     for (int i = 0; i < T1_PRE; ++i) {
       const int idx = NIDX + i * nthr + static_cast<int>(threadIdx.x);
-      if (idx < kLutSize) tab1[idx] = t1_pre[i];
+      if (SINGLE && idx < kLutSize) tab1[idx] = t1_pre[i];
     }
-    for (int idx = NIDX + T1_PRE * nthr + static_cast<int>(threadIdx.x); idx < kLutSize; idx += nthr)
+    for (int idx = NIDX + T1_PRE * nthr + static_cast<int>(threadIdx.x); SINGLE && idx < kLutSize; idx += nthr)
       tab1[idx] = __ldg(M.tab32 + idx);
   } else {
     // [256][32] grid values (entry i of the source in every lane's own bank) and, for the comparator decoder, the
@@ -493,14 +494,14 @@ __device__ __forceinline__ void gemv1_block(const MatDev& M, const Gemv1Args& A,
                                              jj * SPG, jj == 3, acc_a, acc_b);
         finish_sub(jj, acc_a, acc_b);
       }
-    } else if (PAIR_LAYOUT || cls == 0) {   // a pair layout has no other class
+    } else if (ONE_CLASS || cls == 0) {
 #pragma unroll
       for (int jj = 0; jj < NSU; ++jj) {
         int acc_a = 0, acc_b = 0;
         sub_block<G, SPG, MASK, PAIR>(ca, cb, smem, lane_off, xt + jj * SPG, jj * SPG, jj == NSU - 1, acc_a, acc_b);
         finish_sub(jj, acc_a, acc_b);
       }
-    } else if constexpr (!PAIR_LAYOUT) {
+    } else if constexpr (!ONE_CLASS) {
 #pragma unroll
       for (int jj = 0; jj < NSU; ++jj) {
         int acc_a = 0, acc_b = 0;

@@ -35,7 +35,7 @@ static bool plan_gemvm(const MatDev& M, int ntr, GemvmPlan& p) {
   }
   p.max_units = (p.max_units + 1) & ~1;
   if (p.max_units > debug_knobs().max_units) return false;
-  const size_t fixed = (size_t(1) << (M.index_bits + ring_log_copies(M.index_bits) + 2)) + kLutSize * 4 +
+  const size_t fixed = (size_t(1) << (M.index_bits + ring_log_copies(M.index_bits) + 2)) + (one_class(FMT, M.index_bits) ? 0 : kLutSize * 4) +
                        static_cast<size_t>(p.cols_per_set) * (kTileSyms + (has_offset ? 2 : 1) * NSB) * MR * 4 +
                        2 * kGemv1MaxSlots * 8 + kGemv1MaxSlots * 4 + 16 + p.max_units * sizeof(UnitMeta) +
                        kRingSlackWords * 4;
@@ -133,6 +133,7 @@ static int launch_g(const MatDev& M, const void* X, bool x_is_half, int m, float
       if (M.index_bits == 12) return launch_r<FMT, 3, 12>(M, X, x_is_half, m, P, err, st);
     return launch_r<FMT, 3, 11>(M, X, x_is_half, m, P, err, st);
   } else {
+    if (M.index_bits == 9) return launch_r<FMT, 4, 9>(M, X, x_is_half, m, P, err, st);
     switch (M.group) {
       case 3: return launch_i<FMT, 3>(M, X, x_is_half, m, P, err, st);
       case 4: return launch_i<FMT, 4>(M, X, x_is_half, m, P, err, st);

@@ -88,13 +88,14 @@ __global__ void __launch_bounds__(gemvm_threads(MR), 1) k_gemvm(MatDev M, GemvmA
   constexpr bool PAIR_LAYOUT = is_pair_layout(FMT);
   constexpr bool HAS_OFFSET = FMT == kFmtQ4K || FMT == kFmtQ5K || FMT == kFmtQ5KP;
   constexpr int NIDX = 1 << IDXBITS, R = 1 << LOG_R;
-  constexpr bool SINGLE = NIDX <= kLutSize;
+  constexpr bool ONE_CLASS = one_class(FMT, IDXBITS);
+  constexpr bool SINGLE = !ONE_CLASS;   // a single-copy table of all 2048 windows
   constexpr uint32_t MASK = static_cast<uint32_t>(NIDX - 1) << (LOG_R + 2);
   constexpr int kReplicatedTableBytes = NIDX * R * 4;
   extern __shared__ __align__(128) uint8_t smem[];
   uint32_t* tab = reinterpret_cast<uint32_t*>(smem);
   uint32_t* tab1 = reinterpret_cast<uint32_t*>(smem + kReplicatedTableBytes);
-  uint32_t* xq = tab1 + kLutSize;                                                   // [cols][kTileSyms][MR] words
+  uint32_t* xq = tab1 + (SINGLE ? kLutSize : 0);                                                   // [cols][kTileSyms][MR] words
   float* xscale = reinterpret_cast<float*>(xq + static_cast<size_t>(RA.cols_per_set) * kTileSyms * MR);   // [cols][NSB][MR]
   float* xg = xscale + static_cast<size_t>(RA.cols_per_set) * NSB * MR;              // [cols][NSB][MR] (offset formats)
   RingMem RM;
@@ -206,7 +207,7 @@ __global__ void __launch_bounds__(gemvm_threads(MR), 1) k_gemvm(MatDev M, GemvmA
         }
       }
     };
-    if (PAIR_LAYOUT || cls == 0) {   // a pair layout has no other class
+    if (ONE_CLASS || cls == 0) {
 #pragma unroll
       for (int jj = 0; jj < NSU; ++jj) {
         int acc_a[MR], acc_b[MR];
@@ -215,7 +216,7 @@ __global__ void __launch_bounds__(gemvm_threads(MR), 1) k_gemvm(MatDev M, GemvmA
         sub_block_m<G, SPG, MASK, MR>(ca, cb, smem, lane_off, xt + jj * SPG * MR, jj * SPG, jj == NSU - 1, acc_a, acc_b);
         finish_sub(jj, acc_a, acc_b);
       }
-    } else if constexpr (!PAIR_LAYOUT) {
+    } else if constexpr (!ONE_CLASS) {
 #pragma unroll
       for (int jj = 0; jj < 4; ++jj) {
         int acc_a[MR], acc_b[MR];

@@ -31,9 +31,14 @@ constexpr int kRingLogCopies = 4;        // the layout's pad allows up to 16 cop
 #ifndef LW_LOG_COPIES_11
 #define LW_LOG_COPIES_11 3
 #endif
+// A code of at most nine bits (the loader re-codes every block-format matrix with that limit: prepare_matrix) needs 512
+// windows, of which 32 copies fit: every lane has its own copy in its own bank and a lookup is ONE wavefront instead of
+// 2.0 with 16 copies.
 __host__ __device__ constexpr int ring_log_copies(int index_bits) {
-  return index_bits == 12 ? 2 : index_bits == 11 ? LW_LOG_COPIES_11 : kRingLogCopies;   // 64 KB in every case
+  return index_bits == 12 ? 2 : index_bits == 11 ? LW_LOG_COPIES_11 : index_bits == 9 ? 5 : kRingLogCopies;   // 64 KB in every case
 }
+// Instantiations whose reader is exact for any data: no unit classes, hence no single-copy table either.
+__host__ __device__ constexpr bool one_class(int fmt, int index_bits) { return is_pair_layout(fmt) || index_bits == 9; }
 constexpr int kRingMaxWarps = 28;        // consumer warps; up to four more warps produce
 constexpr int kRingMaxSlots = 64;        // staging buffers in the ring
 constexpr int kRingMaxUnits = 1024;      // work units one block can be dealt in one launch
@@ -372,7 +377,7 @@ struct GroupChain {
   // bp0: pad bits to skip.  A chain is laid out with kRingLogCopies + 2 leading zero bits; a kernel whose table has
   // fewer copies (2^LOG_R) wants the window LOG_R + 2 bits up in the shifted word, i.e. starts kRingLogCopies - LOG_R
   // bits into the pad.
-  __device__ __forceinline__ void init(const uint32_t* chain_words, uint32_t bp0 = 0) {
+  __device__ __forceinline__ void init(const uint32_t* chain_words, int bp0 = 0) {
     w0 = chain_words[0];
     w1 = chain_words[32];
     w2 = chain_words[64];
@@ -416,23 +421,27 @@ struct GroupChain {
   }
 };
 
-// The reader of the pair layouts (lw::build_pairs): every group starts by loading its three words from the chain at
-// the word its bit position has reached - no refill, no branch, nothing kept between groups but the position - so a
-// group may use up any number of words.  What remains of the grouping rule is that its last symbol starts within 31
-// bits of its first: always true for groups of three symbols of at most 12 bits.  (Measured on the 11-bit codes of
-// the bundle formats this reader is a few per cent slower than GroupChain: two more shared-memory loads per group.  A
-// variant of GroupChain that holds a fourth word and refills up to twice per group was measured on the pair layout too:
-// 119 M instead of 81 M instructions for eight 14336 x 4096 products, 22.4 instead of 18.3 us each.)
+// The reader of the codes of at most nine bits and of the 12-bit pair layouts (lw::build_pairs): every group starts by
+// loading its three words from the chain at the word its bit position has reached - no refill, no branch, nothing kept
+// between groups but the position - so a group may use up any number of words.  What remains of the grouping rule is
+// that its last symbol starts within 31 bits of its first: always true for four symbols of at most ten bits and for three
+// of at most 12.  A group costs 8 instructions where GroupChain's costs 11 (and GroupChain's groups of paired 4-bit codes
+// hold three symbols, not four), against three shared-memory loads instead of about one, which the conflict-free table
+// pays for: Q4_K, three 14336 x 4096 products in one launch, @@@ us.  (On 11-bit codes under 8 copies of the table
+// this reader is a few per cent slower than GroupChain; a variant of GroupChain that holds a fourth word and refills up to
+// twice per group took 119 M instead of 81 M instructions for eight 14336 x 4096 products of a 12-bit pair layout.)
+// The position may start at -1: with 32 copies the window wants one bit more below it than the chain has pad bits, so the
+// first group reads one bit of the word before the chain (shared memory of the block in any case), which the mask drops.
 struct ReloadChain {
   const uint32_t* base;
-  uint32_t bp;
+  int bp;
   uint32_t a, b, off;
-  __device__ __forceinline__ void init(const uint32_t* chain_words, uint32_t bp0 = 0) {
+  __device__ __forceinline__ void init(const uint32_t* chain_words, int bp0 = 0) {
     base = chain_words;
     bp = bp0;
   }
   __device__ __forceinline__ void begin() {
-    const uint32_t* q = base + (bp >> 5) * 32u;
+    const uint32_t* q = base + (bp & ~31);   // word bp / 32 (rounded down) of the chain: words are 32 apart
     const uint32_t w0 = q[0], w1 = q[32], w2 = q[64];
     a = __funnelshift_r(w0, w1, bp);
     b = __funnelshift_r(w1, w2, bp);
@@ -446,12 +455,6 @@ struct ReloadChain {
     return e;
   }
   __device__ __forceinline__ void end() { bp += off; }
-  __device__ __forceinline__ uint32_t slow_sym(const uint32_t* tab32, uint32_t pad) {
-    const uint32_t* q = base + (bp >> 5) * 32u;
-    const uint32_t e = tab32[(__funnelshift_r(q[0], q[32], bp) >> pad) & (kLutSize - 1)];
-    bp += e >> 28;
-    return e;
-  }
 };
 
 // Pair layouts with an 11-bit code are laid out WITHOUT pad bits: three symbols of at most 11 bits need 33 bits after
@@ -463,7 +466,7 @@ struct ReloadChain2 {
   const uint32_t* base;
   uint32_t bp;
   uint32_t a, b, off;
-  __device__ __forceinline__ void init(const uint32_t* chain_words, uint32_t = 0) {
+  __device__ __forceinline__ void init(const uint32_t* chain_words, int = 0) {
     base = chain_words;
     bp = 0;
   }
@@ -483,18 +486,16 @@ struct ReloadChain2 {
     return e;
   }
   __device__ __forceinline__ void end() { bp += off; }
-  __device__ __forceinline__ uint32_t slow_sym(const uint32_t* tab32, uint32_t) {
-    const uint32_t* q = base + (bp >> 5) * 32u;
-    const uint32_t e = tab32[__funnelshift_r(q[0], q[32], bp) & (kLutSize - 1)];
-    bp += e >> 28;
-    return e;
-  }
 };
 
 // The reader of a kernel instantiation: pair layouts by the width of their code, everything else GroupChain.
 template <bool PAIR_LAYOUT, int IDXBITS>
 struct ChainOf {
   using type = GroupChain;
+};
+template <>
+struct ChainOf<false, 9> {
+  using type = ReloadChain;
 };
 template <>
 struct ChainOf<true, 12> {
