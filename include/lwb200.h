@@ -134,7 +134,7 @@ int lw_matrix_info(void* handle, int id, int* N, int* K, int* fmt, long long* bl
                    long long* device_bytes);
 
 /* How the batch-1 kernel decodes matrix `id` (chosen from the data when the bundle is opened; no reference
- * counterpart): symbols per refill group (0 = that kernel is not used), index bits of its replicated table (10 or 11)
+ * counterpart): symbols per refill group (0 = that kernel is not used), index bits of its replicated table (9, 10 or 11)
  * and the share of work units (64 rows x one column segment) that cannot use that group size and fall back to groups
  * of two symbols or, for 11-bit codes under the 10-bit table, to symbol-by-symbol decoding. */
 int lw_matrix_plan(void* handle, int id, int* group, int* index_bits, double* slow_fraction);
@@ -201,8 +201,8 @@ int lw_decode_codes(void* handle, int id, uint8_t* out_dev, int expand, void* st
 
 /* Builds a one-matrix handle from a blob in host memory (N rows, Ks symbols per row), an optional side tensor and
  * its block format.  The matrix has id 0.  Released by rt_close.
- * What the device holds (here and in rt_open) is the loader's business: a block-format matrix whose code has 11-bit
- * words is re-coded with words of at most 10 bits (LW_RECODE=0 in the environment: not), Q6_K / Q5_K matrices also get a
+ * What the device holds (here and in rt_open) is the loader's business: a block-format matrix whose code has words of
+ * more than nine bits is re-coded with that limit (LW_RECODE=0 in the environment: not), Q6_K / Q5_K matrices also get a
  * pair layout (below).  Decoded symbols, products and the byte counts lw_matrix_info reports for the bundle do not change. */
 void* lw_matrix_create(const uint8_t* blob, long long blob_bytes, int N, int Ks, int fmt, const uint8_t* side,
                        long long side_bytes);
@@ -261,7 +261,7 @@ int lw_host_layout_table(const uint8_t* blob, long long blob_bytes, int N, int K
 /* Pair layout.  For Q6_K and Q5_K matrices whose K is a multiple of 512 the loader keeps a second device layout
  * that every product kernel (one row, 2..8 rows fused, the tensor-core kernel up to 64 rows - where the layout's larger
  * work units fit their shared memory) and the decode to fp16 weights read: two adjacent codes of a row are one symbol of a prefix code built from the matrix's own pair counts (at most
- * 12 bits for pairs of 6-bit codes, 11 for pairs of 5-bit codes), so that the kernel does one table lookup per two
+ * 12 bits for pairs of 6-bit codes, 11 for pairs of 5-bit codes, one less where that costs little), so that the kernel does one table lookup per two
  * weights, as it does for the 4-bit formats whose bundle symbols are pairs already.  The decoded codes are the same;
  * device memory holds the matrix twice (LW_PAIRS=0 in the environment at load: no pair layouts).  No reference
  * counterpart: the reference's kernel decodes these formats one symbol per weight (kernels/llmrt.cu:972-1024).

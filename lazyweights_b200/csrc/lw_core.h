@@ -39,11 +39,13 @@ constexpr int sub_width(int f) { return (f == kFmtQ6K || f == kFmtQ6KP) ? 16 : 3
 constexpr bool is_paired(int f) { return f == kFmtQ4K || f == kFmtIQ4XS || f == kFmtQ6KP || f == kFmtQ5KP; }
 constexpr bool is_pair_layout(int f) { return f == kFmtQ6KP || f == kFmtQ5KP; }
 constexpr int pair_layout_of(int f) { return f == kFmtQ6K ? kFmtQ6KP : f == kFmtQ5K ? kFmtQ5KP : kFmtNone; }
-// Longest code a pair layout's own code may have = index bits of its table: 1024 pairs of 5-bit codes fit 11 bits; the
-// 4096 pairs of 6-bit codes need 12, but a matrix in which at most 2048 different pairs occur gets an 11-bit code where
-// that costs at most a fifth more code bits (the 2048-window table has twice the copies for the same shared memory: fewer
-// bank conflicts per lookup).
+// Longest code a pair layout's own code may have = index bits of its table: 1024 pairs of 5-bit codes fit 11 bits, the
+// 4096 pairs of 6-bit codes need 12; a matrix in which at most half as many code points are used gets a code of one bit
+// less where that costs at most a fifth more code bits (the table of half the windows has twice the copies for the same
+// shared memory: fewer bank conflicts per lookup).
 constexpr int pair_code_bits_max(int f) { return f == kFmtQ6KP ? 12 : 11; }
+constexpr int pair_code_bits_min(int f) { return pair_code_bits_max(f) - 1; }   // where that costs little (lw::build_pairs)
+constexpr int pair_group(int index_bits) { return index_bits == 10 ? 4 : 3; }
 // Column segments per tile row of the device layout: more segments = shorter chains = more of them in flight for the
 // same staging memory; a segment must hold whole quads of sub-blocks (four 32-weight sub-blocks of Q5_K = 128 symbols).
 constexpr int default_split(int f) { return f == kFmtNone ? 1 : f == kFmtQ5K ? 2 : 4; }

@@ -90,6 +90,8 @@ template <int FMT>
 static int launch_i(const MatDev& M, uint8_t* out, bool expand, unsigned int* err, cudaStream_t st) {
   if constexpr (is_pair_layout(FMT)) {
     const int NT = M.N / kTileRows;
+    if constexpr (pair_code_bits_min(FMT) == 10)
+      if (M.index_bits == 10) return launch_t<FMT, 4, 10, true>(M, out, 0, NT, err, st);
     if constexpr (pair_code_bits_max(FMT) == 12)
       if (M.index_bits == 12) return launch_t<FMT, 3, 12, true>(M, out, 0, NT, err, st);
     return launch_t<FMT, 3, 11, true>(M, out, 0, NT, err, st);

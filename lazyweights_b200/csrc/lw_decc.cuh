@@ -61,7 +61,7 @@ __global__ void __launch_bounds__(1024, 1) k_decode_codes_ring(const __grid_cons
   const int nmine = S.nmine;
   ring_reset(RM);
   __syncthreads();
-  ring_build_list<SPLIT>(M, RA, S, RM);
+  ring_build_list<SPLIT, !ONE_CLASS>(M, RA, S, RM);
   __syncthreads();
   if (warp >= RA.warps) {
     ring_produce(M, RA, RM, nmine, warp - RA.warps, lane);

@@ -81,6 +81,8 @@ static int launch_bundle_code(const MatDev& M, __half* out, int tr0, int tr1, un
 template <int FMT>
 static int launch_i(const MatDev& M, __half* out, int tr0, int tr1, unsigned int* err, cudaStream_t st) {
   if constexpr (is_pair_layout(FMT)) {
+    if constexpr (pair_code_bits_min(FMT) == 10)
+      if (M.index_bits == 10) return launch_t<FMT, 4, 10>(M, out, tr0, tr1, err, st);
     if constexpr (pair_code_bits_max(FMT) == 12)
       if (M.index_bits == 12) return launch_t<FMT, 3, 12>(M, out, tr0, tr1, err, st);
     return launch_t<FMT, 3, 11>(M, out, tr0, tr1, err, st);

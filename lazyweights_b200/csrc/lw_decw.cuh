@@ -70,7 +70,7 @@ __global__ void __launch_bounds__(1024, 1) k_decw(const __grid_constant__ MatDev
   // 1. the block's list (whole tiles, symbol-by-symbol tiles first) and the ring's barriers
   ring_reset(RM);
   __syncthreads();
-  ring_build_list<SPLIT>(M, RA, S, RM);
+  ring_build_list<SPLIT, !ONE_CLASS>(M, RA, S, RM);
   __syncthreads();
 
   if (!consumer) {

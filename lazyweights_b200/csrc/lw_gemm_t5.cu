@@ -102,7 +102,9 @@ static int launch_i(const MatDev& M, const __half* X, int m, float* planes, unsi
 template <int FMT>
 static int launch_g(const MatDev& M, const __half* X, int m, float* planes, unsigned int* err, cudaStream_t st,
                     int* terms) {
-  if constexpr (is_pair_layout(FMT)) {   // groups of three pair symbols, the layout's own table
+  if constexpr (is_pair_layout(FMT)) {   // the layout's own table
+    if constexpr (pair_code_bits_min(FMT) == 10)
+      if (M.index_bits == 10) return launch_t<FMT, 4, 10>(M, X, m, planes, err, st, terms);
     if constexpr (pair_code_bits_max(FMT) == 12)
       if (M.index_bits == 12) return launch_t<FMT, 3, 12>(M, X, m, planes, err, st, terms);
     return launch_t<FMT, 3, 11>(M, X, m, planes, err, st, terms);

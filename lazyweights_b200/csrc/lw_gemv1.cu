@@ -181,7 +181,9 @@ static int launch_batch_i(int n, const MatDev* const* mats, const void* const* x
 template <int FMT>
 static int launch_batch_g(int n, const MatDev* const* mats, const void* const* xs, bool x_is_half, float* const* partials,
                           float* const* ys, unsigned int* err, cudaStream_t st) {
-  if constexpr (is_pair_layout(FMT)) {   // groups of three; the table of the layout's own code, 2048 or 4096 windows
+  if constexpr (is_pair_layout(FMT)) {   // the table of the layout's own code
+    if constexpr (pair_code_bits_min(FMT) == 10)
+      if (mats[0]->index_bits == 10) return launch_batch_t<FMT, 4, 10>(n, mats, xs, x_is_half, partials, ys, err, st);
     if constexpr (pair_code_bits_max(FMT) == 12)
       if (mats[0]->index_bits == 12) return launch_batch_t<FMT, 3, 12>(n, mats, xs, x_is_half, partials, ys, err, st);
     return launch_batch_t<FMT, 3, 11>(n, mats, xs, x_is_half, partials, ys, err, st);
@@ -288,6 +290,8 @@ static int launch_i(const MatDev& M, const void* X, bool x_is_half, float* P, fl
 template <int FMT>
 static int launch_g(const MatDev& M, const void* X, bool x_is_half, float* P, float* Y, unsigned int* err, cudaStream_t st) {
   if constexpr (is_pair_layout(FMT)) {
+    if constexpr (pair_code_bits_min(FMT) == 10)
+      if (M.index_bits == 10) return launch_t<FMT, 4, 10, ring_log_copies(10)>(M, X, x_is_half, P, Y, err, st);
     if constexpr (pair_code_bits_max(FMT) == 12)
       if (M.index_bits == 12) return launch_t<FMT, 3, 12, ring_log_copies(12)>(M, X, x_is_half, P, Y, err, st);
     return launch_t<FMT, 3, 11, ring_log_copies(11)>(M, X, x_is_half, P, Y, err, st);
@@ -311,8 +315,8 @@ static int launch_g(const MatDev& M, const void* X, bool x_is_half, float* P, fl
 
 bool gemv1_usable(const MatDev& M) {
   if (is_pair_layout(M.fmt))
-    return (M.index_bits == 11 || M.index_bits == pair_code_bits_max(M.fmt)) && M.pad == pair_pad_bits(M.index_bits) && M.split == default_split(M.fmt) && M.unit_slow && M.row_done &&
-           M.group == 3 && M.reader == 0;
+    return (M.index_bits == pair_code_bits_min(M.fmt) || M.index_bits == pair_code_bits_max(M.fmt)) && M.pad == pair_pad_bits(M.index_bits) && M.split == default_split(M.fmt) && M.unit_slow && M.row_done &&
+           M.group == pair_group(M.index_bits) && M.reader == 0;
   const bool fmt_ok = M.fmt >= kFmtQ4K && M.fmt <= kFmtIQ4XS;
   const int gmax = is_paired(M.fmt) ? 4 : 6;
   return fmt_ok && (M.index_bits == 9 || M.index_bits == 10 || M.index_bits == 11) && M.pad == kRingLogCopies + 2 && M.split == default_split(M.fmt) && M.unit_slow && M.row_done && M.group >= 3 &&

@@ -225,6 +225,37 @@ static __device__ __noinline__ void row_sum(const float* p, unsigned int terms, 
   if (lane < 16) reinterpret_cast<float4*>(y)[lane] = acc;
 }
 
+// Eight consecutive activations as floats; 16-byte loads where the address allows them (the same answer for every thread of
+// a launch: rows start at multiples of eight values).
+__device__ __forceinline__ void load_x8(const void* x, int is_half, size_t at, float (&v)[8]) {
+  const bool wide = (reinterpret_cast<uintptr_t>(x) & 15u) == 0;
+  if (is_half) {
+    const __half* h = static_cast<const __half*>(x) + at;
+    __align__(16) __half2 p[4];
+    if (wide) {
+      *reinterpret_cast<uint4*>(p) = *reinterpret_cast<const uint4*>(h);
+    } else {
+#pragma unroll
+      for (int i = 0; i < 4; ++i) p[i] = __halves2half2(h[2 * i], h[2 * i + 1]);
+    }
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+      const float2 f = __half22float2(p[i]);
+      v[2 * i] = f.x;
+      v[2 * i + 1] = f.y;
+    }
+  } else {
+    const float* f = static_cast<const float*>(x) + at;
+    if (wide) {
+      const float4 a = *reinterpret_cast<const float4*>(f), b = *reinterpret_cast<const float4*>(f + 4);
+      v[0] = a.x, v[1] = a.y, v[2] = a.z, v[3] = a.w, v[4] = b.x, v[5] = b.y, v[6] = b.z, v[7] = b.w;
+    } else {
+#pragma unroll
+      for (int i = 0; i < 8; ++i) v[i] = f[i];
+    }
+  }
+}
+
 #ifdef LW_GEMV1_PROFILE
 // Built with -DLW_GEMV1_PROFILE, every consumer warp adds up the clock cycles it spends in the phases of its loop; the
 // sums over all warps land here: [0] prologue, [1] drawing a unit and waiting for its copy, [2] decoding, [3] handing
@@ -278,52 +309,17 @@ __device__ __forceinline__ void gemv1_block(const MatDev& M, const Gemv1Args& A,
   const bool consumer = warp < A.helpers;   // takes part in the prologue; warps >= RA.warps leave after it
   const int nthr = A.helpers * 32;
 
-  // 1. everything the prologue needs from global memory is requested at once: table entries and the first activations
-  // (consumers), then where the block's units live (all threads)
-  // The registers stay exactly as loaded until after the barriers below: converting or moving one earlier would make
-  // the warp wait for its load right here.
-  constexpr int TAB_PRE = 3, T1_PRE = 2, XB = 6;
-  uint32_t tab_pre[TAB_PRE], t1_pre[T1_PRE], xraw[XB];
-  auto load_x = [&](int base) {
-#pragma unroll
-    for (int u = 0; u < XB; ++u) {
-      const int i = base + u * nthr + threadIdx.x;
-      xraw[u] = 0u;
-      if (i < ncol * TW) {
-        const int j = i / TW, k = i - j * TW;
-        const size_t src = static_cast<size_t>(set + RA.nsets * j) * TW + k;
-        if (A.x_is_half)
-          xraw[u] = static_cast<const unsigned short*>(A.x)[src];
-        else
-          xraw[u] = static_cast<const uint32_t*>(A.x)[src];
-      }
-    }
-  };
-  auto x_value = [&](uint32_t raw) {
-    return A.x_is_half ? __half2float(__ushort_as_half(static_cast<unsigned short>(raw))) : __uint_as_float(raw);
-  };
-  if (consumer) {
-    if (READER == kReaderTable) {
-#pragma unroll
-      for (int i = 0; i < TAB_PRE; ++i) {
-        const int idx = (i * A.helpers + warp) * 32 + lane;
-        tab_pre[i] = idx < NIDX ? __ldg(M.tab32 + idx) : 0u;
-      }
-#pragma unroll
-      for (int i = 0; i < T1_PRE; ++i) {   // windows beyond the replicated table (single-copy table only)
-        const int idx = NIDX + i * nthr + static_cast<int>(threadIdx.x);
-        t1_pre[i] = SINGLE && idx < kLutSize ? __ldg(M.tab32 + idx) : 0u;
-      }
-    }
-    if (!A.pdl) load_x(0);
-  }
+  // 1. the table's entries are requested at once, then where the block's units live (all threads).  The registers stay
+  // exactly as loaded until after the barriers below: touching one earlier would make the warp wait for its load there.
+  TableLoad<IDXBITS, LOG_R, SINGLE> table;
+  if (READER == kReaderTable) table.issue(M.tab32, warp, lane, A.helpers);
   if (threadIdx.x < ring) {
     tile_cnt[threadIdx.x] = 0u;
     tile_free[threadIdx.x] = 0u;
   }
   ring_reset(RM);
   __syncthreads();
-  ring_build_list<SPLIT>(M, RA, S, RM);
+  ring_build_list<SPLIT, !ONE_CLASS>(M, RA, S, RM);
   __syncthreads();
 
   if (!consumer) {
@@ -334,20 +330,7 @@ __device__ __forceinline__ void gemv1_block(const MatDev& M, const Gemv1Args& A,
   // 2b. consumers: table and activations (the first copies are already on their way).
   uint32_t lim[10] = {0u, 0u, 0u, 0u, 0u, 0u, 0u, 0u, 0u, 0u};
   if (READER == kReaderTable) {
-#pragma unroll
-    for (int i = 0; i < TAB_PRE; ++i) {
-      const int i0 = (i * A.helpers + warp) * 32;
-      if (i0 < NIDX) table_spread<LOG_R, SINGLE>(tab, tab1, i0, tab_pre[i], lane);
-    }
-    for (int i0 = (TAB_PRE * A.helpers + warp) * 32; i0 < NIDX; i0 += A.helpers * 32)
-      table_spread<LOG_R, SINGLE>(tab, tab1, i0, __ldg(M.tab32 + i0 + lane), lane);
-#pragma unroll
-    for (int i = 0; i < T1_PRE; ++i) {
-      const int idx = NIDX + i * nthr + static_cast<int>(threadIdx.x);
-      if (SINGLE && idx < kLutSize) tab1[idx] = t1_pre[i];
-    }
-    for (int idx = NIDX + T1_PRE * nthr + static_cast<int>(threadIdx.x); SINGLE && idx < kLutSize; idx += nthr)
-      tab1[idx] = __ldg(M.tab32 + idx);
+    if (consumer) table.finish(M.tab32, tab, tab1, warp, lane, A.helpers);
   } else {
     // [256][32] grid values (entry i of the source in every lane's own bank) and, for the comparator decoder, the
     // [12][32] offsets behind them and the ten limits in registers
@@ -363,33 +346,41 @@ __device__ __forceinline__ void gemv1_block(const MatDev& M, const Gemv1Args& A,
   // Everything up to here read only the matrix (tables, list, and the producers' copies of chain words): with a
   // programmatic launch it overlaps the tail of the previous kernel in the stream, which may still be writing x.
   if (A.pdl) pdl_wait();
-  // activations -> 16-bit fixed point with one scale per sub-block (GW consecutive weights sit in GW consecutive
-  // lanes).  Loads go out XB at a time so that their global-memory latencies overlap.
-  for (int base = 0; base < ncol * TW; base += XB * nthr) {
-    if (base > 0 || A.pdl) load_x(base);
+  // Activations -> 16-bit fixed point with one scale per sub-block.  A thread takes eight consecutive weights (one 16-byte
+  // load of fp16 values, two of fp32): a sub-block is two or four neighbouring lanes, so its maximum and sum cost one or
+  // two shuffles per eight values.  (With one value per thread the shuffles - eleven per value - took 3300 cycles of every
+  // block, as long as decoding a unit.)
+  constexpr int LPS = GW / 8;   // lanes per sub-block
+  for (int c = threadIdx.x; c < ncol * (TW / 8); c += nthr) {   // whole sub-blocks take the loop together: TW / 8 is a multiple of 32
+    const int j = c / (TW / 8), k = (c - j * (TW / 8)) * 8;
+    const size_t src = static_cast<size_t>(set + RA.nsets * j) * TW + k;
+    float v[8];
+    load_x8(A.x, A.x_is_half, src, v);
+    float amax = 0.f, sum = 0.f;
 #pragma unroll
-    for (int u = 0; u < XB; ++u) {
-      const int i = base + u * nthr + threadIdx.x;
-      if (i < ncol * TW) {   // whole warps take this branch together: sizes are multiples of 32
-        const float xvu = x_value(xraw[u]);
-        float amax = fabsf(xvu), sum = xvu;
+    for (int i = 0; i < 8; ++i) {
+      amax = fmaxf(amax, fabsf(v[i]));
+      sum += v[i];
+    }
 #pragma unroll
-        for (int o = 1; o < GW; o <<= 1) {
-          amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, o));
-          if (HAS_OFFSET) sum += __shfl_xor_sync(0xffffffffu, sum, o);
-        }
-        const int q = __float2int_rn(xvu * (amax > 0.f ? 32767.f / amax : 0.f));
-        if (PAIR) {
-          const int qn = __shfl_down_sync(0xffffffffu, q, 1);
-          if ((lane & 1) == 0) xq[i >> 1] = (static_cast<uint32_t>(q) & 0xFFFFu) | (static_cast<uint32_t>(qn) << 16);
-        } else {
-          xq[i] = static_cast<uint32_t>(q);   // sign-extended: the operand of a 32-bit multiply-add
-        }
-        if ((lane & (GW - 1)) == 0) {
-          xscale[i / GW] = amax * (1.f / 32767.f);
-          if (HAS_OFFSET) xg[i / GW] = sum;
-        }
-      }
+    for (int o = 1; o < LPS; o <<= 1) {
+      amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, o));
+      if (HAS_OFFSET) sum += __shfl_xor_sync(0xffffffffu, sum, o);
+    }
+    const float to_int = amax > 0.f ? 32767.f / amax : 0.f;
+    uint32_t q[8];
+#pragma unroll
+    for (int i = 0; i < 8; ++i) q[i] = static_cast<uint32_t>(__float2int_rn(v[i] * to_int));
+    if (PAIR) {   // a word per paired symbol
+      *reinterpret_cast<uint4*>(xq + c * 4) = make_uint4(__byte_perm(q[0], q[1], 0x5410), __byte_perm(q[2], q[3], 0x5410),
+                                                         __byte_perm(q[4], q[5], 0x5410), __byte_perm(q[6], q[7], 0x5410));
+    } else {      // a word per weight, sign-extended: the operand of a 32-bit multiply-add
+      *reinterpret_cast<uint4*>(xq + c * 8) = make_uint4(q[0], q[1], q[2], q[3]);
+      *reinterpret_cast<uint4*>(xq + c * 8 + 4) = make_uint4(q[4], q[5], q[6], q[7]);
+    }
+    if (c % LPS == 0) {
+      xscale[c / LPS] = amax * (1.f / 32767.f);
+      if (HAS_OFFSET) xg[c / LPS] = sum;
     }
   }
   asm volatile("bar.sync 1, %0;" ::"r"(nthr) : "memory");

@@ -128,7 +128,9 @@ static int launch_i(const MatDev& M, const void* X, bool x_is_half, int m, float
 
 template <int FMT>
 static int launch_g(const MatDev& M, const void* X, bool x_is_half, int m, float* P, unsigned int* err, cudaStream_t st) {
-  if constexpr (is_pair_layout(FMT)) {   // groups of three pair symbols, the layout's own table
+  if constexpr (is_pair_layout(FMT)) {   // the layout's own table
+    if constexpr (pair_code_bits_min(FMT) == 10)
+      if (M.index_bits == 10) return launch_r<FMT, 4, 10>(M, X, x_is_half, m, P, err, st);
     if constexpr (pair_code_bits_max(FMT) == 12)
       if (M.index_bits == 12) return launch_r<FMT, 3, 12>(M, X, x_is_half, m, P, err, st);
     return launch_r<FMT, 3, 11>(M, X, x_is_half, m, P, err, st);

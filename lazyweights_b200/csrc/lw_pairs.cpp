@@ -148,33 +148,33 @@ int build_pairs(const uint8_t* sym, int N, int K, int fmt, const uint8_t* side, 
   // 2. the pair code: limited lengths, canonical codes (shorter first, then by symbol), stream order LSB first
   std::vector<uint8_t> len;
   limited_lengths_n(counts, L, len);
-  if (L == 12) {
-    // 11 bits where no more than 2048 pairs occur and the shorter limit costs at most `slack` per cent of code bits
-    // (LW_PAIR_SLACK, default 20): the 2048-window table has 8 copies instead of 4 in the same shared memory, a
-    // lookup costs 2.6 instead of 3.8 shared-memory wavefronts and products run 10 % faster (the kernel is bound by
-    // shared memory, not by DRAM: measured with 16 % more code bits, 18.3 instead of 20.1 us).
-    static const int slack = [] {
-      const char* e = getenv("LW_PAIR_SLACK");
-      return e ? std::max(0, std::min(100, atoi(e))) : 20;
-    }();
-    size_t used = 0;
-    for (int64_t c : counts) used += c > 0;
-    if (used <= 2048) {
-      std::vector<uint8_t> len11;
-      limited_lengths_n(counts, 11, len11);
-      int64_t bits12 = 0, bits11 = 0;
-      for (int p = 0; p < NP; ++p) {
-        bits12 += counts[p] * len[p];
-        bits11 += counts[p] * len11[p];
-      }
-      if (bits11 * 100 <= bits12 * (100 + slack)) {
-        len.swap(len11);
-        L = 11;
-      }
+  // A shorter limit where no more pairs occur than it has code points and it costs at most `slack` per cent of code bits
+  // (LW_PAIR_SLACK, default 20): the table of half the windows has twice the copies in the same shared memory, which is
+  // what bounds the kernels, not DRAM.  Q6_K 12 -> 11 bits: 3.3 instead of 3.8 shared-memory wavefronts per lookup, 18.3
+  // instead of 20.1 us for a 14336 x 4096 product at 16 % more code bits.  Q5_K 11 -> 10 bits: 2.0 instead of 3.3
+  // wavefronts, and groups of four symbols instead of three.
+  static const int slack = [] {
+    const char* e = getenv("LW_PAIR_SLACK");
+    return e ? std::max(0, std::min(100, atoi(e))) : 20;
+  }();
+  auto code_bits = [&](const std::vector<uint8_t>& l) {
+    int64_t bits = 0;
+    for (int p = 0; p < NP; ++p) bits += counts[p] * l[p];
+    return bits;
+  };
+  size_t used = 0;
+  for (int64_t c : counts) used += c > 0;
+  if (used <= (size_t(1) << (L - 1))) {
+    std::vector<uint8_t> shorter;
+    limited_lengths_n(counts, L - 1, shorter);
+    if (code_bits(shorter) * 100 <= code_bits(len) * (100 + slack)) {
+      len.swap(shorter);
+      --L;
     }
   }
   out.index_bits = L;
-  // an 11-bit code is laid out without pad bits (its reader loads two words per group: lw_ring.cuh), a 12-bit code
+  out.group = pair_group(L);   // symbols per group: the last one starts within 31 bits of the first
+  // an 11-bit code is laid out without pad bits (its reader loads two words per group: lw_ring.cuh), the others
   // with the six the table's address bits want
   const int pad = L == 11 ? 0 : 6;
   out.pad = pad;

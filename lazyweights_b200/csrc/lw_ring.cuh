@@ -136,7 +136,8 @@ __device__ __forceinline__ void ring_reset(const RingMem& R) {
 // hold a symbol-by-symbol unit moved to the front (such a unit takes several times longer: started last, it would keep
 // the whole block waiting).  The order within the two classes is whatever the counters hand out; results do not depend
 // on it.  Also initialises the barriers of the ring.  All threads of the block call this between two __syncthreads.
-template <int SPLIT>
+// CLASSES = false (readers that are exact for any data): the tiles stay in order, nothing is asked about them.
+template <int SPLIT, bool CLASSES = true>
 __device__ __forceinline__ void ring_build_list(const MatDev& M, const RingArgs& A, const BlockShare& S,
                                                 const RingMem& R) {
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -156,23 +157,28 @@ __device__ __forceinline__ void ring_build_list(const MatDev& M, const RingArgs&
       g0 = __ldg(gb);
       g1 = __ldg(gb + 1);
       g2 = __ldg(gb + 2);
-      const uint8_t* uc = M.unit_slow + static_cast<size_t>(t) * SPLIT;
-      cls = __ldg(uc + seg);
+      if (CLASSES) {
+        const uint8_t* uc = M.unit_slow + static_cast<size_t>(t) * SPLIT;
+        cls = __ldg(uc + seg);
 #pragma unroll
-      for (int i = 0; i < SPLIT; ++i) slow |= __ldg(uc + i) == 2;
+        for (int i = 0; i < SPLIT; ++i) slow |= __ldg(uc + i) == 2;
+      }
     }
-    const uint32_t bs = __ballot_sync(0xffffffffu, valid && leader && slow);
-    const uint32_t bf = __ballot_sync(0xffffffffu, valid && leader && !slow);
-    int base_s = 0, base_f = 0;
-    if (lane == 0) {
-      base_s = atomicAdd(list_count, __popc(bs));
-      base_f = atomicAdd(list_count + 1, __popc(bf));
+    int tpos = k / SPLIT;
+    if constexpr (CLASSES) {
+      const uint32_t bs = __ballot_sync(0xffffffffu, valid && leader && slow);
+      const uint32_t bf = __ballot_sync(0xffffffffu, valid && leader && !slow);
+      int base_s = 0, base_f = 0;
+      if (lane == 0) {
+        base_s = atomicAdd(list_count, __popc(bs));
+        base_f = atomicAdd(list_count + 1, __popc(bf));
+      }
+      base_s = __shfl_sync(0xffffffffu, base_s, 0);
+      base_f = __shfl_sync(0xffffffffu, base_f, 0);
+      const uint32_t below = (1u << lane) - 1u;
+      tpos = slow ? base_s + __popc(bs & below) : S.tmine - 1 - (base_f + __popc(bf & below));
+      tpos = __shfl_sync(0xffffffffu, tpos, lane - seg);   // the tile's position, from its leader
     }
-    base_s = __shfl_sync(0xffffffffu, base_s, 0);
-    base_f = __shfl_sync(0xffffffffu, base_f, 0);
-    const uint32_t below = (1u << lane) - 1u;
-    int tpos = slow ? base_s + __popc(bs & below) : S.tmine - 1 - (base_f + __popc(bf & below));
-    tpos = __shfl_sync(0xffffffffu, tpos, lane - seg);   // the tile's position, from its leader
     if (valid) {
       const int pos = tpos * SPLIT + seg;
       R.meta[pos] = UnitMeta{g0,
@@ -265,55 +271,39 @@ __device__ __forceinline__ void ring_release(const RingMem& R, const Unit& u, in
 // (lane % R) << 2.  Every chain starts with pad = LOG_R + 2 zero bits, which puts the window on exactly those address
 // bits of the funnel-shifted word: the entry address is one three-input logic operation.
 //
-// Spreads 32 entries held by a warp (lane l holds entry i0 + l): broadcast one by one, every lane stores its own copy
-// (bank = lane, no conflicts).  With 16 copies two entries go out per store.  tab1 = the single-copy table.
-template <int LOG_R, bool SINGLE = true>
-__device__ __forceinline__ void table_spread(uint32_t* tab, uint32_t* tab1, int i0, uint32_t mine, int lane) {
-  constexpr int R = 1 << LOG_R, PER = 32 / R;   // entries per store: lane l writes copy l % R of entry i0 + j + l / R
-#pragma unroll 8
-  for (int j = 0; j < 32; j += PER) {
-    const uint32_t v = __shfl_sync(0xffffffffu, mine, j + (lane >> LOG_R));
-    tab[(i0 + j) * R + lane] = v;
-  }
-  if (SINGLE) tab1[i0 + lane] = mine;
-}
-
-// The whole table, by `nwarps` warps (warp, lane = the caller's position among them).  SINGLE = false: no single-copy
-// table (a kernel whose replicated table already holds all 2048 windows has no use for it).
-template <int IDXBITS, int LOG_R, bool SINGLE = true>
-__device__ __forceinline__ void table_fill(const MatDev& M, uint32_t* tab, uint32_t* tab1, int warp, int lane,
-                                           int nwarps) {
-  constexpr int NIDX = 1 << IDXBITS;
-  for (int i0 = warp * 32; i0 < NIDX; i0 += nwarps * 32)
-    table_spread<LOG_R, SINGLE>(tab, tab1, i0, __ldg(M.tab32 + i0 + lane), lane);
-  if (SINGLE)
-    for (int idx = NIDX + warp * 32 + lane; idx < kLutSize; idx += nwarps * 32) tab1[idx] = __ldg(M.tab32 + idx);
-}
-
-// The same in two steps, for kernels that have set-up to do between them: issue() starts up to PRE loads per lane right
-// at the kernel's start (their latency, a DRAM miss for the first block that touches the table, then overlaps the unit
-// list's own loads and barriers), finish() spreads them and loads whatever a small block has left.
-template <int IDXBITS, int LOG_R, bool SINGLE = true, int PRE = 8>
+// The R copies of a window are one contiguous row of R * 4 bytes, all the same word: R / 4 lanes write a row with 16-byte
+// stores, so a warp's store fills 128 / R windows, its lanes having loaded just those entries (neighbouring lanes the same
+// one).  64 KB of table are 128 loads and 128 stores for the block.  (The first form loaded 32 entries per warp and handed
+// them round with a shuffle per store: 512 shuffles and 512 4-byte stores, which share one issue port: 1750 cycles of the
+// 12400 that a one-row product of a 1024 x 4096 matrix spends in a block; this form about 300.)  issue() starts up to PRE loads
+// per lane right at the kernel's start, so that their latency (a DRAM miss for the first block that touches the table)
+// overlaps the unit list's own loads and barriers; finish() stores them and loads what a small block has left.
+// SINGLE: also the single-copy table of all 2048 windows (tab1), for the units decoded symbol by symbol.
+template <int IDXBITS, int LOG_R, bool SINGLE, int PRE = 5>
 struct TableLoad {
-  static constexpr int NIDX = 1 << IDXBITS;
+  static constexpr int NIDX = 1 << IDXBITS, LPW = (1 << LOG_R) / 4, WPS = 32 / LPW, STORES = NIDX / WPS;
+  static_assert(LOG_R >= 2, "a copy row is a whole number of 16-byte pieces");
   uint32_t pre[PRE];
   __device__ __forceinline__ void issue(const uint32_t* src, int warp, int lane, int nwarps) {
 #pragma unroll
     for (int i = 0; i < PRE; ++i) {
-      const int i0 = (i * nwarps + warp) * 32;
-      pre[i] = warp < nwarps && i0 < NIDX ? __ldg(src + i0 + lane) : 0u;
+      const int s = i * nwarps + warp;
+      pre[i] = warp < nwarps && s < STORES ? __ldg(src + s * WPS + lane / LPW) : 0u;
     }
   }
   __device__ __forceinline__ void finish(const uint32_t* src, uint32_t* tab, uint32_t* tab1, int warp, int lane, int nwarps) const {
+    uint4* rows = reinterpret_cast<uint4*>(tab) + lane;
 #pragma unroll
     for (int i = 0; i < PRE; ++i) {
-      const int i0 = (i * nwarps + warp) * 32;
-      if (i0 < NIDX) table_spread<LOG_R, SINGLE>(tab, tab1, i0, pre[i], lane);
+      const int s = i * nwarps + warp;
+      if (s < STORES) rows[s * 32] = make_uint4(pre[i], pre[i], pre[i], pre[i]);
     }
-    for (int i0 = (PRE * nwarps + warp) * 32; i0 < NIDX; i0 += nwarps * 32)
-      table_spread<LOG_R, SINGLE>(tab, tab1, i0, __ldg(src + i0 + lane), lane);
+    for (int s = PRE * nwarps + warp; s < STORES; s += nwarps) {
+      const uint32_t v = __ldg(src + s * WPS + lane / LPW);
+      rows[s * 32] = make_uint4(v, v, v, v);
+    }
     if (SINGLE)
-      for (int idx = NIDX + warp * 32 + lane; idx < kLutSize; idx += nwarps * 32) tab1[idx] = __ldg(src + idx);
+      for (int idx = warp * 32 + lane; idx < kLutSize; idx += nwarps * 32) tab1[idx] = __ldg(src + idx);
   }
 };
 
@@ -421,13 +411,13 @@ struct GroupChain {
   }
 };
 
-// The reader of the codes of at most nine bits and of the 12-bit pair layouts (lw::build_pairs): every group starts by
+// The reader of the codes of at most nine bits and of the 10- and 12-bit pair layouts (lw::build_pairs): every group starts by
 // loading its three words from the chain at the word its bit position has reached - no refill, no branch, nothing kept
 // between groups but the position - so a group may use up any number of words.  What remains of the grouping rule is
 // that its last symbol starts within 31 bits of its first: always true for four symbols of at most ten bits and for three
 // of at most 12.  A group costs 8 instructions where GroupChain's costs 11 (and GroupChain's groups of paired 4-bit codes
 // hold three symbols, not four), against three shared-memory loads instead of about one, which the conflict-free table
-// pays for: Q4_K, three 14336 x 4096 products in one launch, @@@ us.  (On 11-bit codes under 8 copies of the table
+// pays for: Q4_K, three 14336 x 4096 products in one launch, 44.5 instead of 49.5 us.  (On 11-bit codes under 8 copies of the table
 // this reader is a few per cent slower than GroupChain; a variant of GroupChain that holds a fourth word and refills up to
 // twice per group took 119 M instead of 81 M instructions for eight 14336 x 4096 products of a 12-bit pair layout.)
 // The position may start at -1: with 32 copies the window wants one bit more below it than the chain has pad bits, so the
@@ -495,6 +485,10 @@ struct ChainOf {
 };
 template <>
 struct ChainOf<false, 9> {
+  using type = ReloadChain;
+};
+template <>
+struct ChainOf<true, 10> {
   using type = ReloadChain;
 };
 template <>

@@ -49,3 +49,22 @@ def test_decode_and_gemm(lw, ty, n, k, rows, half):
                 z = torch.empty(m * k + 1, device="cuda")
                 z[1:] = torch.from_numpy(x).cuda().reshape(-1)
                 assert torch.equal(mat.linear("m", z[1:].reshape(m, k)), torch.from_numpy(y[:m]).cuda())
+
+
+# Q5_K pair layouts: narrow codes get a 10-bit pair code (groups of four), codes all over the range an 11-bit one
+@pytest.mark.parametrize("n,k,wide", [(64, 512, False), (192, 1536, False), (256, 2048, True)])
+def test_q5k_pair_code_lengths(lw, n, k, wide):
+    import torch
+    q, side, sym, w, rng = helpers.seeded_case("Q5_K", n, k, seed=n * 3 + k)
+    if wide:
+        q[:16] = rng.integers(0, 32, (16, k), dtype=np.uint8)   # nearly every pair occurs: ten bits would be a fixed width
+        sym, w = orc.symbols_of("Q5_K", q), orc.dequant("Q5_K", q, side)
+    assert lw.bundle.host_pairs(q, "Q5_K", side)["index_bits"] == (11 if wide else 10)
+    blob, _, _ = lw.bundle.encode_huf8(sym)
+    with lw.CodedMatrix(blob, n, k, "Q5_K", side) as mat:
+        assert np.array_equal(mat.decode_codes("m").cpu().numpy(), q)
+        assert np.array_equal(mat.decode_weights("m").cpu().numpy().view(np.uint16), w.astype(np.float16).view(np.uint16))
+        for m in (1, 3, 8, 20):
+            x = rng.standard_normal((m, k)).astype(np.float32)
+            y = mat.linear("m", torch.from_numpy(x).cuda()).cpu().numpy()
+            assert helpers.rel_err(y, orc.gemv_f64(w, x)) <= TOL, m
