@@ -152,7 +152,8 @@ int build_pairs(const uint8_t* sym, int N, int K, int fmt, const uint8_t* side, 
   // (LW_PAIR_SLACK, default 20): the table of half the windows has twice the copies in the same shared memory, which is
   // what bounds the kernels, not DRAM.  Q6_K 12 -> 11 bits: 3.3 instead of 3.8 shared-memory wavefronts per lookup, 18.3
   // instead of 20.1 us for a 14336 x 4096 product at 16 % more code bits.  Q5_K 11 -> 10 bits: 2.0 instead of 3.3
-  // wavefronts, and groups of four symbols instead of three.
+  // wavefronts, groups of four symbols instead of three, but three words loaded per group instead of two: taken up to half
+  // the slack (pairs of Gaussian codes cost 4.6 per cent; pairs from all over the range 15 to 25).
   static const int slack = [] {
     const char* e = getenv("LW_PAIR_SLACK");
     return e ? std::max(0, std::min(100, atoi(e))) : 20;
@@ -167,7 +168,7 @@ int build_pairs(const uint8_t* sym, int N, int K, int fmt, const uint8_t* side, 
   if (used <= (size_t(1) << (L - 1))) {
     std::vector<uint8_t> shorter;
     limited_lengths_n(counts, L - 1, shorter);
-    if (code_bits(shorter) * 100 <= code_bits(len) * (100 + slack)) {
+    if (code_bits(shorter) * 100 <= code_bits(len) * (100 + (L - 1 == 10 ? slack / 2 : slack))) {
       len.swap(shorter);
       --L;
     }
