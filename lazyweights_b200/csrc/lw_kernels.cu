@@ -631,6 +631,21 @@ static void launch_dependent(void (*kernel)(KArgs...), dim3 grid, dim3 block, cu
   cudaLaunchKernelEx(&cfg, kernel, static_cast<KArgs>(args)...);
 }
 
+// dst = src, n 16-byte pieces read straight out of (pinned) host memory.  For small activations this replaces a copy on a
+// copy engine, whose hand-over to the product kernel costs more than the bytes; the product is a programmatic dependent, so
+// its set-up (table, unit list, first weights) runs while the pieces cross PCIe.
+__global__ void __launch_bounds__(256) k_pull(const uint4* __restrict__ src, uint4* __restrict__ dst, int n) {
+  pdl_trigger();
+  const int i = blockIdx.x * 256 + threadIdx.x;
+  if (i < n) dst[i] = src[i];
+}
+
+int launch_pull(const void* host_src, void* dst, size_t bytes, cudaStream_t st) {
+  const int n = static_cast<int>((bytes + 15) / 16);
+  k_pull<<<(n + 255) / 256, 256, 0, st>>>(static_cast<const uint4*>(host_src), static_cast<uint4*>(dst), n);
+  return check_launch("k_pull");
+}
+
 int launch_rows_to_half(const float* src, __half* dst, int m, int K, float* scales, cudaStream_t st) {
   launch_dependent(k_rows_to_half, dim3(m), dim3(kToHalfThreads), st, src, dst, K, m, scales);
   return check_launch("k_rows_to_half");

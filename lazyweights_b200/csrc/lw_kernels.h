@@ -45,6 +45,8 @@ int launch_decode_codes(const MatDev& M, uint8_t* out, bool expand_pairs, cudaSt
 int launch_decode_weights(const MatDev& M, __half* out, cudaStream_t st);
 // Only tile rows tr0 .. tr1 - 1 (64 matrix rows each); `out` receives those rows, [ (tr1 - tr0) * 64, K ].
 int launch_decode_weights_rows(const MatDev& M, __half* out, int tr0, int tr1, cudaStream_t st);
+// dst = the bytes (rounded up to 16) at a 16-byte aligned address of pinned host memory, by a kernel.
+int launch_pull(const void* host_src, void* dst, size_t bytes, cudaStream_t st);
 // fp32 activations on their way to fp16: dst = half(src * scales[r]) with scales[r] = a power of two that brings row r
 // inside fp16's range (1 unless the row holds values above 2^15), scales[m + r] = its inverse, to be applied to row r of
 // the product.

@@ -27,6 +27,11 @@ def _torch():
     return torch
 
 
+def _stream(torch, device_index):
+    """The current stream's handle (torch.cuda.current_stream builds an object around it first: 1.5 us)."""
+    return torch._C._cuda_getCurrentRawStream(device_index)
+
+
 class _Handle:
     def __init__(self, ptr):
         if not ptr:
@@ -34,10 +39,12 @@ class _Handle:
         self._h = C.c_void_p(ptr)
         self._ids = {}
         self._info = {}
+        self._linear = {}
 
     # ---- lifetime
     def close(self):
         if self._h:
+            self._linear = {}   # they hold the handle
             nat.lib().rt_close(self._h)
             self._h = None
 
@@ -82,18 +89,26 @@ class _Handle:
     # ---- device-pointer path
     def linear(self, name, x, out=None):
         """x: CUDA tensor [m, K] or [K], fp16 or fp32 -> fp32 [m, N] (or [N])."""
+        # A small product takes 6 us on the GPU, so this wrapper counts: look-ups are kept, plain integers go to ctypes.
         torch = _torch()
-        inf = self.info(name)
-        squeeze = x.dim() == 1
-        x2 = x.reshape(1, -1) if squeeze else x
-        if not x2.is_cuda or x2.dtype not in (torch.float16, torch.float32) or x2.shape[1] != inf["K"]:
-            raise ValueError("linear wants a CUDA fp16/fp32 tensor with %d columns" % inf["K"])
-        x2 = x2.contiguous()
-        m = x2.shape[0]
-        y = out if out is not None else torch.empty((m, inf["N"]), dtype=torch.float32, device=x2.device)
-        st = torch.cuda.current_stream(x2.device).cuda_stream
-        nat.check(nat.lib().lw_linear(self._h, self.matrix_id(name), C.c_void_p(x2.data_ptr()),
-                                      int(x2.dtype == torch.float16), m, C.c_void_p(y.data_ptr()), C.c_void_p(st)))
+        known = self._linear.get(name)
+        if known is None:
+            inf = self.info(name)
+            known = self._linear[name] = (self._h.value if self._h else None, self.matrix_id(name), inf["N"], inf["K"])
+        handle, mid, n, k = known
+        shape, half = x.shape, x.dtype is torch.float16
+        if not x.is_cuda or not (half or x.dtype is torch.float32) or shape[-1] != k:
+            raise ValueError("linear wants a CUDA fp16/fp32 tensor with %d columns" % k)
+        if len(shape) > 2:
+            raise ValueError("linear wants one or two dimensions")
+        squeeze = len(shape) == 1
+        m = 1 if squeeze else shape[0]
+        if not x.is_contiguous():
+            x = x.contiguous()
+        y = out if out is not None else torch.empty((m, n), dtype=torch.float32, device=x.device)
+        rc = nat.lib().lw_linear(handle, mid, x.data_ptr(), half, m, y.data_ptr(), _stream(torch, x.get_device()))
+        if rc < 0:
+            nat.check(rc)
         return y[0] if squeeze and out is None else y
 
     def linear_static(self, name, x, out):
@@ -147,8 +162,7 @@ class _Handle:
         w = out if out is not None else torch.empty((inf["N"], inf["K"]), dtype=torch.float16, device="cuda")
         if w.dtype != torch.float16 or tuple(w.shape) != (inf["N"], inf["K"]) or not w.is_cuda or not w.is_contiguous():
             raise ValueError("decode_weights wants a contiguous CUDA fp16 [%d, %d] tensor" % (inf["N"], inf["K"]))
-        st = torch.cuda.current_stream().cuda_stream
-        nat.check(nat.lib().lw_decode_weights(self._h, self.matrix_id(name), C.c_void_p(w.data_ptr()), C.c_void_p(st)))
+        nat.check(nat.lib().lw_decode_weights(self._h, self.matrix_id(name), w.data_ptr(), _stream(torch, torch.cuda.current_device())))
         return w
 
     def decode_codes(self, name, expand=True, out=None):
@@ -161,20 +175,23 @@ class _Handle:
             out = torch.empty((inf["N"], cols), dtype=torch.uint8, device="cuda")
         if out.dtype != torch.uint8 or tuple(out.shape) != (inf["N"], cols) or not out.is_cuda or not out.is_contiguous():
             raise ValueError("decode_codes wants a contiguous CUDA uint8 [%d, %d] tensor" % (inf["N"], cols))
-        st = torch.cuda.current_stream().cuda_stream
-        nat.check(nat.lib().lw_decode_codes(self._h, self.matrix_id(name), C.c_void_p(out.data_ptr()), int(expand),
-                                            C.c_void_p(st)))
+        nat.check(nat.lib().lw_decode_codes(self._h, self.matrix_id(name), out.data_ptr(), int(expand),
+                                            _stream(torch, torch.cuda.current_device())))
         return out
 
     # ---- host-buffer path (reference-named entry points)
     def matmul(self, name, X, path=0):
         """Y[m, N] = X[m, K] . W^T with host float32 arrays (rt_test_matmul)."""
-        X = np.ascontiguousarray(np.atleast_2d(X), np.float32)
-        inf = self.info(name)
+        X = np.ascontiguousarray(X, np.float32)
+        if X.ndim != 2:
+            X = np.atleast_2d(X)
+        inf = self._info.get(name) or self.info(name)
         if X.shape[1] != inf["K"]:
             raise ValueError("X has %d columns, the matrix %d" % (X.shape[1], inf["K"]))
         Y = np.empty((X.shape[0], inf["N"]), np.float32)
-        nat.check(nat.lib().rt_test_matmul(self._h, name.encode(), _address(X), X.shape[0], _address(Y), path))
+        rc = nat.lib().rt_test_matmul(self._h, name.encode(), _address(X), X.shape[0], _address(Y), path)
+        if rc < 0:
+            nat.check(rc)
         return Y
 
     def decode(self, name):
@@ -215,8 +232,9 @@ class ProductBatch:
             self._xs[j], self._ys[j] = x.data_ptr(), y.data_ptr()
 
     def launch(self):
-        st = _torch().cuda.current_stream().cuda_stream
-        nat.check(nat.lib().lw_linear_batch(self._n, self._handles, self._ids, self._xs, self._half, self._ys, C.c_void_p(st)))
+        torch = _torch()
+        nat.check(nat.lib().lw_linear_batch(self._n, self._handles, self._ids, self._xs, self._half, self._ys,
+                                            _stream(torch, torch.cuda.current_device())))
 
 
 class Bundle(_Handle):
