@@ -854,11 +854,11 @@ int rt_test_matmul(void* handle, const char* name, const float* X, int m, float*
     M->pin_floats = nx + ny;
   }
   std::memcpy(M->h_pin, X, nx * 4);
-  // Up to 256 KB a kernel fetches them (IQ4_XS 8192 x 3072, one row: 28.1 instead of 29.6 us per call); beyond, a copy engine moves more per
-  // microsecond than the copy's hand-over costs.
+  // One row is fetched by a kernel (IQ4_XS 8192 x 3072: 28.1 instead of 29.6 us per call), several rows by a copy engine: their
+  // products start with launches that have less set-up to hide the fetch behind.  The kernel may only run on the model's device.
   int rc = kOk;
-  if (nx * 4 <= (size_t(256) << 10)) {
-    if ((rc = launch_pull(M->h_pin, M->d_x, nx * 4, nullptr))) return rc;
+  if (m == 1 && nx * 4 <= (size_t(256) << 10)) {
+    if ((rc = check_device(M)) || (rc = launch_pull(M->h_pin, M->d_x, nx * 4, nullptr))) return rc;
   } else if ((e = cudaMemcpyAsync(M->d_x, M->h_pin, nx * 4, cudaMemcpyHostToDevice, nullptr)) != cudaSuccess) {
     return cuda_fail("rt_test_matmul copy in", e);
   }

@@ -97,11 +97,9 @@ class _Handle:
             known = self._linear[name] = (self._h.value if self._h else None, self.matrix_id(name), inf["N"], inf["K"])
         handle, mid, n, k = known
         shape, half = x.shape, x.dtype is torch.float16
-        if not x.is_cuda or not (half or x.dtype is torch.float32) or shape[-1] != k:
-            raise ValueError("linear wants a CUDA fp16/fp32 tensor with %d columns" % k)
-        if len(shape) > 2:
-            raise ValueError("linear wants one or two dimensions")
         squeeze = len(shape) == 1
+        if not x.is_cuda or not (half or x.dtype is torch.float32) or shape[0 if squeeze else 1] != k:
+            raise ValueError("linear wants a CUDA fp16/fp32 tensor with %d columns" % k)
         m = 1 if squeeze else shape[0]
         if not x.is_contiguous():
             x = x.contiguous()
