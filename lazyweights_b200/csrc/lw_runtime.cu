@@ -21,6 +21,7 @@
 
 #include "../../include/lwb200.h"
 #include "lw_model.h"
+#include "lw_gemv1.h"
 
 namespace lw {
 
@@ -559,6 +560,253 @@ __global__ void __launch_bounds__(kAttnThreads)
   }
 }
 
+// The same attention for passes of several tokens.  A block of k_attn serves one token, so a pass of m tokens read every key
+// and value m times and staged them m times: 252 us for 64 tokens at a context of 2048 (8 kv heads, 4 query heads each),
+// 48.7 us for 8 tokens at 1008 (32 kv heads).  Here a block serves a tile of R = 8 RW query rows of one kv head - row r of the
+// pass is head r % group of token r / group - so a chunk is read once per tile; bound: fp32 multiply-adds from about 16 rows
+// on, below that the latency of the chunks' loads.
+//  * A warp owns RW rows for the whole kernel: its scores, running maximum, sum and outputs stay in registers, and nothing
+//    but the staged chunk is shared between warps.  Lane l holds the scores of positions l and l + 32 of the chunk and, in
+//    the value phase, dimensions 4 l .. 4 l + 3.  Per eight dimensions a warp reads 16 wavefronts of keys and queries for
+//    64 RW / 4 multiply-adds: at RW = 4 both pipes are equally busy.
+//  * A block walks a span of chunks with the running-maximum rescaling.  While it works on keys the values of the chunk are on
+//    their way into registers, while it works on values the next chunk's keys are.
+//  * Spans: as many per tile as bring two blocks to every SM; their results are merged in span order by the block that is last
+//    (the counter of k_attn).  Chunks per span follow from the position on the device, so a captured pass covers any of its bucket.
+// Queries, scores, probabilities and sums are fp32, as in k_attn.
+constexpr int kRowsStride = kAttnMaxDh / 2 + 4;   // words per staged row: 16-byte aligned, 8 lanes' 16-byte loads hit 32 banks
+constexpr int kRowsMaxSpans = 32;                  // a lane of the merge holds one span
+
+template <int RW>
+__global__ void __launch_bounds__(kAttnThreads, 2)
+    k_attn_rows(const float* __restrict__ qkv, const __half* __restrict__ kc, const __half* __restrict__ vc,
+                float* __restrict__ part, float* __restrict__ att, unsigned int* __restrict__ done,
+                const int* __restrict__ posp, int m, int H, int Hk, int Dh, int Tmax, float scale, int window, int max_chunks) {
+  dep_begin();
+  constexpr int R = kAttnThreads / 32 * RW;
+  __shared__ __align__(16) uint32_t kv[kAttnChunk * kRowsStride];
+  __shared__ __align__(16) float qs[R][kAttnMaxDh];
+  __shared__ __align__(16) float ps[R][kAttnChunk];
+  __shared__ unsigned int s_last;
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int group = H / Hk, rows = m * group, kh = blockIdx.x, r0 = blockIdx.y * R, spans = gridDim.z, pos = *posp;
+  const int t_first = r0 / group, t_last = (min(rows, r0 + R) - 1) / group;
+  const int hi = pos + t_last + 1, lo = window > 0 ? max(0, pos + t_first - window + 1) : 0;   // positions any row of the tile sees
+  const int total = (hi - lo + kAttnChunk - 1) / kAttnChunk, per = (total + spans - 1) / spans;
+  const int c0 = blockIdx.z * per, c1 = min(total, c0 + per);
+  // this warp's rows: token, head, first and last position they see (rows past the end see nothing)
+  const int row0 = r0 + warp * RW;
+  int first[RW], last[RW], all_first = 0, all_last = 0x7fffffff;
+#pragma unroll
+  for (int i = 0; i < RW; ++i) {
+    const int t = (row0 + i) / group;
+    last[i] = row0 + i < rows ? pos + t : -1;
+    first[i] = window > 0 ? max(0, pos + t - window + 1) : 0;
+    if (row0 + i < rows) {
+      all_first = max(all_first, first[i]);
+      all_last = min(all_last, last[i]);
+    }
+  }
+  for (int i = threadIdx.x; i < R * (Dh / 4); i += kAttnThreads) {
+    const int r = i / (Dh / 4), d = (i - r * (Dh / 4)) * 4, g = r0 + r;
+    float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
+    if (g < rows)
+      v = *reinterpret_cast<const float4*>(qkv + static_cast<size_t>(g / group) * (H + 2 * Hk) * Dh + static_cast<size_t>(kh * group + g % group) * Dh + d);
+    *reinterpret_cast<float4*>(&qs[r][d]) = v;
+  }
+  const int cpr = Dh / 8;                                              // 16-byte pieces per row
+  constexpr int VPT = kAttnChunk * (kAttnMaxDh / 8) / kAttnThreads;    // pieces per thread (4)
+  auto fetch = [&](const __half* base, int c, uint4 (&reg)[VPT]) {
+    const int p0 = lo + c * kAttnChunk, n = min(kAttnChunk, hi - p0);
+    const __half* src = base + (static_cast<size_t>(kh) * Tmax + p0) * Dh;
+#pragma unroll
+    for (int u = 0; u < VPT; ++u) {
+      const int idx = threadIdx.x + u * kAttnThreads, t = idx / cpr, ch = idx - t * cpr;
+      reg[u] = make_uint4(0u, 0u, 0u, 0u);
+      if (idx < kAttnChunk * cpr && t < n) reg[u] = __ldg(reinterpret_cast<const uint4*>(src + static_cast<size_t>(t) * Dh) + ch);
+    }
+  };
+  auto place = [&](const uint4 (&reg)[VPT]) {
+#pragma unroll
+    for (int u = 0; u < VPT; ++u) {
+      const int idx = threadIdx.x + u * kAttnThreads, t = idx / cpr, ch = idx - t * cpr;
+      if (idx < kAttnChunk * cpr) *reinterpret_cast<uint4*>(kv + t * kRowsStride + ch * 4) = reg[u];
+    }
+  };
+  float mx[RW], sum[RW], out[RW][4];
+#pragma unroll
+  for (int i = 0; i < RW; ++i) {
+    mx[i] = -INFINITY;
+    sum[i] = 0.f;
+#pragma unroll
+    for (int d = 0; d < 4; ++d) out[i][d] = 0.f;
+  }
+  const bool mine = row0 < rows;
+  uint4 kreg[VPT], vreg[VPT];
+  if (c0 < c1) fetch(kc, c0, kreg);
+  for (int c = c0; c < c1; ++c) {
+    __syncthreads();   // the values of the chunk before have been read (first time: nothing)
+    place(kreg);
+    fetch(vc, c, vreg);
+    __syncthreads();
+    const int p0 = lo + c * kAttnChunk;
+    float s[RW][2];
+    if (mine) {
+#pragma unroll
+      for (int i = 0; i < RW; ++i) s[i][0] = s[i][1] = 0.f;
+      const uint32_t* ka = kv + lane * kRowsStride;
+      const uint32_t* kb = ka + 32 * kRowsStride;
+#pragma unroll 2
+      for (int d = 0; d < Dh; d += 8) {
+        const uint4 a = *reinterpret_cast<const uint4*>(ka + d / 2), b = *reinterpret_cast<const uint4*>(kb + d / 2);
+        const uint32_t aw[4] = {a.x, a.y, a.z, a.w}, bw[4] = {b.x, b.y, b.z, b.w};
+        float2 af[4], bf[4];
+#pragma unroll
+        for (int w = 0; w < 4; ++w) {
+          af[w] = __half22float2(*reinterpret_cast<const __half2*>(aw + w));
+          bf[w] = __half22float2(*reinterpret_cast<const __half2*>(bw + w));
+        }
+#pragma unroll
+        for (int i = 0; i < RW; ++i) {
+          const float4 q0 = *reinterpret_cast<const float4*>(&qs[warp * RW + i][d]), q1 = *reinterpret_cast<const float4*>(&qs[warp * RW + i][d + 4]);
+          s[i][0] = fmaf(q0.x, af[0].x, s[i][0]);
+          s[i][1] = fmaf(q0.x, bf[0].x, s[i][1]);
+          s[i][0] = fmaf(q0.y, af[0].y, s[i][0]);
+          s[i][1] = fmaf(q0.y, bf[0].y, s[i][1]);
+          s[i][0] = fmaf(q0.z, af[1].x, s[i][0]);
+          s[i][1] = fmaf(q0.z, bf[1].x, s[i][1]);
+          s[i][0] = fmaf(q0.w, af[1].y, s[i][0]);
+          s[i][1] = fmaf(q0.w, bf[1].y, s[i][1]);
+          s[i][0] = fmaf(q1.x, af[2].x, s[i][0]);
+          s[i][1] = fmaf(q1.x, bf[2].x, s[i][1]);
+          s[i][0] = fmaf(q1.y, af[2].y, s[i][0]);
+          s[i][1] = fmaf(q1.y, bf[2].y, s[i][1]);
+          s[i][0] = fmaf(q1.z, af[3].x, s[i][0]);
+          s[i][1] = fmaf(q1.z, bf[3].x, s[i][1]);
+          s[i][0] = fmaf(q1.w, af[3].y, s[i][0]);
+          s[i][1] = fmaf(q1.w, bf[3].y, s[i][1]);
+        }
+      }
+#pragma unroll
+      for (int i = 0; i < RW; ++i) {
+        const bool va = p0 + lane >= first[i] && p0 + lane <= last[i], vb = p0 + lane + 32 >= first[i] && p0 + lane + 32 <= last[i];
+        const float sa = va ? s[i][0] * scale : -INFINITY, sb = vb ? s[i][1] * scale : -INFINITY;
+        float top = fmaxf(mx[i], fmaxf(sa, sb));
+        for (int o = 16; o; o >>= 1) top = fmaxf(top, __shfl_xor_sync(0xffffffffu, top, o));
+        const float ea = va ? __expf(sa - top) : 0.f, eb = vb ? __expf(sb - top) : 0.f;
+        const float keep = sum[i] == 0.f ? 0.f : __expf(mx[i] - top);   // nothing so far: its maximum is -inf, and so may the new one be
+        ps[warp * RW + i][lane] = ea;
+        ps[warp * RW + i][lane + 32] = eb;
+        float es = ea + eb;
+        for (int o = 16; o; o >>= 1) es += __shfl_xor_sync(0xffffffffu, es, o);
+        sum[i] = sum[i] * keep + es;
+        mx[i] = top;
+#pragma unroll
+        for (int d = 0; d < 4; ++d) out[i][d] *= keep;
+      }
+    }
+    __syncthreads();   // the keys have been read
+    place(vreg);
+    if (c + 1 < c1) fetch(kc, c + 1, kreg);
+    __syncthreads();
+    if (mine && lane * 4 < Dh) {
+      const uint32_t* vcol = kv + lane * 2;
+      const int n = min(kAttnChunk, hi - p0);
+#pragma unroll 2
+      for (int p = 0; p < n; p += 4) {
+        float4 w[RW];
+#pragma unroll
+        for (int i = 0; i < RW; ++i) w[i] = *reinterpret_cast<const float4*>(&ps[warp * RW + i][p]);
+        // positions that only some rows see are not multiplied into the others: a weight of zero would not hide an infinity
+        const bool every = p0 + p >= all_first && p0 + p + 3 <= all_last;
+#pragma unroll
+        for (int k = 0; k < 4; ++k) {
+          const uint2 v = *reinterpret_cast<const uint2*>(vcol + (p + k) * kRowsStride);
+          const float2 x = __half22float2(*reinterpret_cast<const __half2*>(&v.x)), y = __half22float2(*reinterpret_cast<const __half2*>(&v.y));
+#pragma unroll
+          for (int i = 0; i < RW; ++i) {
+            const float wk = k == 0 ? w[i].x : k == 1 ? w[i].y : k == 2 ? w[i].z : w[i].w;
+            if (every || (p0 + p + k >= first[i] && p0 + p + k <= last[i])) {   // the same for the whole warp
+              out[i][0] = fmaf(wk, x.x, out[i][0]);
+              out[i][1] = fmaf(wk, x.y, out[i][1]);
+              out[i][2] = fmaf(wk, y.x, out[i][2]);
+              out[i][3] = fmaf(wk, y.y, out[i][3]);
+            }
+          }
+        }
+      }
+    }
+  }
+  auto result = [&](int i) {   // where row i of this warp goes
+    const int g = row0 + i;
+    return reinterpret_cast<float4*>(att + static_cast<size_t>(g / group) * H * Dh + static_cast<size_t>(kh * group + g % group) * Dh) + lane;
+  };
+  if (spans == 1) {
+#pragma unroll
+    for (int i = 0; i < RW; ++i)
+      if (row0 + i < rows && lane * 4 < Dh)
+        *result(i) = make_float4(out[i][0] / sum[i], out[i][1] / sum[i], out[i][2] / sum[i], out[i][3] / sum[i]);
+    return;
+  }
+  auto span_of = [&](int i, int z) { return part + ((static_cast<size_t>(row0 + i) * Hk + kh) * max_chunks + z) * (Dh + 2); };
+#pragma unroll
+  for (int i = 0; i < RW; ++i)
+    if (row0 + i < rows) {
+      float2* p = reinterpret_cast<float2*>(span_of(i, blockIdx.z));
+      if (lane == 0) p[0] = make_float2(mx[i], sum[i]);
+      if (lane * 4 < Dh) {
+        p[1 + 2 * lane] = make_float2(out[i][0], out[i][1]);
+        p[2 + 2 * lane] = make_float2(out[i][2], out[i][3]);
+      }
+    }
+  __threadfence();
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    unsigned int* cnt = done + static_cast<size_t>(blockIdx.y) * Hk + kh;
+    const unsigned int old = atomicAdd(cnt, 1u);
+    s_last = old == static_cast<unsigned int>(spans) - 1u ? 1u : 0u;
+    if (s_last) *cnt = 0u;   // ready for the next pass
+  }
+  __syncthreads();
+  if (!s_last) return;
+  __threadfence();
+#pragma unroll 1
+  for (int i = 0; i < RW; ++i) {
+    if (row0 + i >= rows) break;
+    float2 ms = make_float2(-INFINITY, 0.f);
+    if (lane < spans) ms = __ldcg(reinterpret_cast<const float2*>(span_of(i, lane)));
+    float top = ms.x;
+    for (int o = 16; o; o >>= 1) top = fmaxf(top, __shfl_xor_sync(0xffffffffu, top, o));
+    const float w = ms.y == 0.f ? 0.f : __expf(ms.x - top);   // a span that saw no position weighs nothing
+    float tot = ms.y * w;
+    for (int o = 16; o; o >>= 1) tot += __shfl_xor_sync(0xffffffffu, tot, o);
+    float4 acc = make_float4(0.f, 0.f, 0.f, 0.f);
+    for (int z0 = 0; z0 < spans; z0 += 8) {
+      float2 x[8], y[8];
+#pragma unroll
+      for (int u = 0; u < 8; ++u) {
+        x[u] = y[u] = make_float2(0.f, 0.f);
+        if (z0 + u < spans && lane * 4 < Dh) {
+          const float2* p = reinterpret_cast<const float2*>(span_of(i, z0 + u));
+          x[u] = __ldcg(p + 1 + 2 * lane);
+          y[u] = __ldcg(p + 2 + 2 * lane);
+        }
+      }
+#pragma unroll
+      for (int u = 0; u < 8; ++u) {   // in span order
+        const float wz = __shfl_sync(0xffffffffu, w, (z0 + u) & 31);
+        if (z0 + u < spans) {
+          acc.x = fmaf(wz, x[u].x, acc.x);
+          acc.y = fmaf(wz, x[u].y, acc.y);
+          acc.z = fmaf(wz, y[u].x, acc.z);
+          acc.w = fmaf(wz, y[u].y, acc.w);
+        }
+      }
+    }
+    if (lane * 4 < Dh) *result(i) = make_float4(acc.x / tot, acc.y / tot, acc.z / tot, acc.w / tot);
+  }
+}
+
 // Greedy decoding on the device: the id of the largest logit (the lowest id among equals, like a host arg-max) becomes
 // the next pass's token, the position advances, the token is appended to the list of generated tokens.  logits: one row;
 // with W ranks the rank-major gather of their slices (slot r: Vmax floats, the first (base + (r < rem)) * 64 valid, ids
@@ -931,14 +1179,21 @@ static int enqueue_pass(Model* M, Runtime* R, int m, bool all_logits, int nchunk
                                                           R->Tmax);
     {
       const int group = R->H / R->Hk;
-      if (group % 4 == 0)
-        launch_dep(k_attn<4>, dim3(R->H / 4, m, nchunks), dim3(kAttnThreads), st, R->qkv, kc, vc, R->attn_part, R->att, R->attn_done,
+      if (m > 1) {   // tiles of 8, 16 or 32 query rows per kv head
+        const int rows = m * group, rw = rows > 16 ? 4 : rows > 8 ? 2 : 1, tiles = (rows + 8 * rw - 1) / (8 * rw);
+        const int want = std::min({nchunks, kRowsMaxSpans, (2 * sm_count() + R->Hk * tiles - 1) / (R->Hk * tiles)});
+        const int per = (nchunks + want - 1) / want, spans = (nchunks + per - 1) / per;
+        launch_dep(rw == 4 ? k_attn_rows<4> : rw == 2 ? k_attn_rows<2> : k_attn_rows<1>, dim3(R->Hk, tiles, spans), dim3(kAttnThreads), st,
+                   R->qkv, kc, vc, R->attn_part, R->att, R->attn_done, posp, m, R->H, R->Hk, R->Dh, R->Tmax, R->attn_scale, R->window,
+                   R->max_chunks);
+      } else if (group % 4 == 0)
+        launch_dep(k_attn<4>, dim3(R->H / 4, 1, nchunks), dim3(kAttnThreads), st, R->qkv, kc, vc, R->attn_part, R->att, R->attn_done,
                    posp, R->H, R->Hk, R->Dh, R->Tmax, R->attn_scale, R->window, R->max_chunks);
       else if (group % 2 == 0)
-        launch_dep(k_attn<2>, dim3(R->H / 2, m, nchunks), dim3(kAttnThreads), st, R->qkv, kc, vc, R->attn_part, R->att, R->attn_done,
+        launch_dep(k_attn<2>, dim3(R->H / 2, 1, nchunks), dim3(kAttnThreads), st, R->qkv, kc, vc, R->attn_part, R->att, R->attn_done,
                    posp, R->H, R->Hk, R->Dh, R->Tmax, R->attn_scale, R->window, R->max_chunks);
       else
-        launch_dep(k_attn<1>, dim3(R->H, m, nchunks), dim3(kAttnThreads), st, R->qkv, kc, vc, R->attn_part, R->att, R->attn_done,
+        launch_dep(k_attn<1>, dim3(R->H, 1, nchunks), dim3(kAttnThreads), st, R->qkv, kc, vc, R->attn_part, R->att, R->attn_done,
                    posp, R->H, R->Hk, R->Dh, R->Tmax, R->attn_scale, R->window, R->max_chunks);
     }
     if ((rc = linear_device(M, M->mats[R->m_o[l]], R->att, false, m, R->o, R->D, st))) return rc;
