@@ -232,23 +232,29 @@ __global__ void __launch_bounds__(kToHalfThreads)
   for (int k = kToHalfHeld * kToHalfThreads + threadIdx.x; k < quads; k += kToHalfThreads) out[k] = halves(load(k));
 }
 
-// Y[j, n] = sum over the `terms` partial rows of P[term, j, n], added in term order (no atomics: results do not
-// depend on scheduling).  One thread per four consecutive outputs: 16-byte loads, eight terms in flight.
+// Y[j, n] = sum over the `terms` partial rows of P[term, j, n], in a fixed order (no atomics: results do not depend on
+// scheduling).  Four consecutive outputs per thread, PARTS threads per four outputs: part p adds terms p, p + PARTS, ...,
+// then the parts are added with shuffles.  What bounds it is the chain of round trips to L2, one per eight terms of a thread:
+// with one part, 64 terms (the down projection of eight tokens, 8 x 3072 outputs) took 20 us, 24 terms 8 us
+// (now about 5 and 4: a 32-layer pass of eight tokens 5.49 -> 4.30 ms; Q6_K 14336 x 4096, eight rows, 49.6 -> 40.5 us).
 // unscale (may be null): factor per output row j, applied to the finished sum.
-__global__ void k_sum_partials(const float* __restrict__ P, float* __restrict__ Y, int m, int N, int ldy, int terms,
-                               const float* __restrict__ unscale = nullptr) {
+template <int PARTS>
+__global__ void __launch_bounds__(128) k_sum_partials(const float* __restrict__ P, float* __restrict__ Y, int m, int N, int ldy, int terms,
+                                                      const float* __restrict__ unscale) {
   pdl_trigger();   // launched as a programmatic dependent of the kernel that writes P (see lw_device.cuh)
   pdl_wait();
-  const int quads = N / 4, i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= m * quads) return;
-  const int j = i / quads, n = (i - j * quads) * 4;
+  constexpr int QW = 32 / PARTS;   // groups of four outputs per warp: neighbouring lanes, so that a part's loads are contiguous
+  const int quads = N / 4, lane = threadIdx.x & 31, part = lane / QW;
+  const int i = (blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5)) * QW + lane % QW;
+  const bool valid = i < m * quads;
+  const int j = valid ? i / quads : 0, n = valid ? (i - j * quads) * 4 : 0;
   const float4* p = reinterpret_cast<const float4*>(P + static_cast<size_t>(j) * N + n);
   const size_t stride = static_cast<size_t>(m) * quads;   // one term further, in float4
   float4 acc = make_float4(0.f, 0.f, 0.f, 0.f);
-  for (int t0 = 0; t0 < terms; t0 += 8) {
+  for (int t0 = part; t0 < terms; t0 += 8 * PARTS) {
     float4 v[8];
 #pragma unroll
-    for (int u = 0; u < 8; ++u) v[u] = t0 + u < terms ? __ldg(p + (t0 + u) * stride) : make_float4(0.f, 0.f, 0.f, 0.f);
+    for (int u = 0; u < 8; ++u) v[u] = t0 + u * PARTS < terms ? __ldg(p + (t0 + u * PARTS) * stride) : make_float4(0.f, 0.f, 0.f, 0.f);
 #pragma unroll
     for (int u = 0; u < 8; ++u) {
       acc.x += v[u].x;
@@ -257,6 +263,14 @@ __global__ void k_sum_partials(const float* __restrict__ P, float* __restrict__ 
       acc.w += v[u].w;
     }
   }
+#pragma unroll
+  for (int o = QW; o < 32; o <<= 1) {
+    acc.x += __shfl_xor_sync(0xffffffffu, acc.x, o);
+    acc.y += __shfl_xor_sync(0xffffffffu, acc.y, o);
+    acc.z += __shfl_xor_sync(0xffffffffu, acc.z, o);
+    acc.w += __shfl_xor_sync(0xffffffffu, acc.w, o);
+  }
+  if (!valid || part > 0) return;
   if (unscale) {
     const float f = unscale[j];
     acc.x *= f;
@@ -270,6 +284,10 @@ __global__ void k_sum_partials(const float* __restrict__ P, float* __restrict__ 
   y[2] = acc.z;
   y[3] = acc.w;
 }
+
+// One round trip of eight loads per thread, up to 64 terms.
+static int sum_parts(int terms) { return terms > 32 ? 8 : terms > 8 ? 4 : 1; }
+static auto sum_kernel(int parts) { return parts == 8 ? k_sum_partials<8> : parts == 4 ? k_sum_partials<4> : k_sum_partials<1>; }
 
 // ------------------------------------------------------------------------------------------------------ launchers
 
@@ -480,7 +498,8 @@ int launch_gemv(const MatDev& M, const void* X, bool x_is_half, int m, float* Y,
   const int terms = M.KT * M.split;
   {
     cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3((m * (M.N / 4) + 127) / 128);
+    const int parts = sum_parts(terms);
+    cfg.gridDim = dim3((m * (M.N / 4) + 128 / parts - 1) / (128 / parts));
     cfg.blockDim = dim3(128);
     // more shared memory than the product kernel leaves free: blocks of the sum that move in beside it and wait there cost
     // it 6 % (Q6_K 14336 x 4096, 8 rows: 52.5 instead of 49.6 us with the sum)
@@ -493,7 +512,7 @@ int launch_gemv(const MatDev& M, const void* X, bool x_is_half, int m, float* Y,
     // measured: waiting early pays for small products (Q4_K 4096 x 4096, 8 rows: 26 -> 20 us) and costs on large ones
     // (Q6_K 14336 x 4096, 8 rows: 78 -> 88 us), so only up to 16 MB of partial products
     cfg.numAttrs = static_cast<size_t>(terms) * m * M.N * 4 <= (size_t(16) << 20) ? 1 : 0;
-    cudaLaunchKernelEx(&cfg, k_sum_partials, static_cast<const float*>(partials), Y, m, M.N, ldy, terms,
+    cudaLaunchKernelEx(&cfg, sum_kernel(parts), static_cast<const float*>(partials), Y, m, M.N, ldy, terms,
                        static_cast<const float*>(nullptr));
   }
   return check_launch("k_sum_partials");
@@ -652,7 +671,8 @@ int launch_rows_to_half(const float* src, __half* dst, int m, int K, float* scal
 }
 
 int launch_sum_partials(const float* P, float* Y, int m, int N, int ldy, int terms, const float* unscale, cudaStream_t st) {
-  launch_dependent(k_sum_partials, dim3((m * (N / 4) + 127) / 128), dim3(128), st, P, Y, m, N, ldy, terms, unscale);
+  const int parts = sum_parts(terms), per_block = 128 / parts;
+  launch_dependent(sum_kernel(parts), dim3((m * (N / 4) + per_block - 1) / per_block), dim3(128), st, P, Y, m, N, ldy, terms, unscale);
   return check_launch("k_sum_partials");
 }
 
