@@ -298,9 +298,15 @@ struct TableLoad {
       const int s = i * nwarps + warp;
       if (s < STORES) rows[s * 32] = make_uint4(pre[i], pre[i], pre[i], pre[i]);
     }
-    for (int s = PRE * nwarps + warp; s < STORES; s += nwarps) {
-      const uint32_t v = __ldg(src + s * WPS + lane / LPW);
-      rows[s * 32] = make_uint4(v, v, v, v);
+    // what is left in a block of few warps (a matrix of few tiles), eight loads in flight at a time:
+    // one after the other they made the decode of 256 x 1024 Q5_K codes 12.5 us, against 8.4
+    for (int s0 = PRE * nwarps + warp; s0 < STORES; s0 += 8 * nwarps) {
+      uint32_t v[8];
+#pragma unroll
+      for (int i = 0; i < 8; ++i) v[i] = s0 + i * nwarps < STORES ? __ldg(src + (s0 + i * nwarps) * WPS + lane / LPW) : 0u;
+#pragma unroll
+      for (int i = 0; i < 8; ++i)
+        if (s0 + i * nwarps < STORES) rows[(s0 + i * nwarps) * 32] = make_uint4(v[i], v[i], v[i], v[i]);
     }
     if (SINGLE)
       for (int idx = warp * 32 + lane; idx < kLutSize; idx += nwarps * 32) tab1[idx] = __ldg(src + idx);
