@@ -56,7 +56,17 @@ static int launch_o(const MatDev& M, __half* out, int tr0, int tr1, unsigned int
   a.r.tr0 = tr0;
   a.r.ntr = tr1 - tr0;
   a.out = out;
-  kernel<<<blocks, (warps + 2) * 32, smem, st>>>(M, a, tm);
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3(blocks);
+  cfg.blockDim = dim3((warps + 2) * 32);
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = st;
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[0].val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = 1;
+  cudaLaunchKernelEx(&cfg, kernel, M, a, tm);
   return note_launch("k_decw");
 }
 

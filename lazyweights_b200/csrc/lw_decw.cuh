@@ -66,6 +66,7 @@ __global__ void __launch_bounds__(1024, 1) k_decw(const __grid_constant__ MatDev
   const int nmine = S.nmine;
   const bool consumer = warp < RA.warps;
   const int nthr = RA.warps * 32;
+  pdl_trigger();   // see lw_gemv1.cuh: the set-up reads only the matrix and overlaps the previous kernel's tail
 
   // 1. the block's list (whole tiles, symbol-by-symbol tiles first) and the ring's barriers
   ring_reset(RM);
@@ -80,6 +81,7 @@ __global__ void __launch_bounds__(1024, 1) k_decw(const __grid_constant__ MatDev
 
   // 2b. consumers: the tables
   table.finish(M.tab32, tab, tab1, warp, lane, RA.warps);
+  pdl_wait();      // `out` may still be read: by the product over the rows that were decoded into it before
   asm volatile("bar.sync 1, %0;" ::"r"(nthr) : "memory");
   const uint32_t lane_off = (lane & (R - 1)) << 2;
   WarpTileStage stage;

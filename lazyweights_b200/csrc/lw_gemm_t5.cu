@@ -83,7 +83,17 @@ static int launch_t(const MatDev& M, const __half* X, int m, float* planes, unsi
   a.r.max_units = p.max_units;
   a.r.tr0 = 0;
   a.r.ntr = M.N / kTileRows;
-  kernel<<<p.blocks, kT5Threads, p.smem, st>>>(M, a);
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3(p.blocks);
+  cfg.blockDim = dim3(kT5Threads);
+  cfg.dynamicSmemBytes = p.smem;
+  cfg.stream = st;
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[0].val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = 1;
+  cudaLaunchKernelEx(&cfg, kernel, M, a);
   *terms = p.nsets;
   return note_launch("k_gemm_t5");
 }

@@ -100,6 +100,7 @@ __global__ void __launch_bounds__(kT5Threads, 1) k_gemm_t5(const __grid_constant
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   TableLoad<IDXBITS, LOG_R, SINGLE> table;
   table.issue(M.tab32, warp, lane, kT5Consumers);
+  pdl_trigger();   // the set-up, up to the activations, reads only the matrix and overlaps the previous kernel's tail
   const int NT = M.N / kTileRows, NRG = NT / 4;                   // row groups of four tile rows
   const int set = blockIdx.x % RA.nsets, bi = blockIdx.x / RA.nsets;
   const int nb_set = (gridDim.x - set + RA.nsets - 1) / RA.nsets;
@@ -154,8 +155,10 @@ __global__ void __launch_bounds__(kT5Threads, 1) k_gemm_t5(const __grid_constant
     ring_produce(M, RA, RM, nmine, warp - kT5Consumers, lane);        // ---- producers: the staging ring
   }
 
+  if (warp < kT5Consumers) table.finish(M.tab32, tab, tab1, warp, lane, kT5Consumers);
   // ---- X in the canonical K-major layout (all warps but the producers, which are already copying)
   if (warp < kT5Consumers || warp == kT5Consumers + kT5Producers) {
+    pdl_wait();   // the activations come from the kernel before, and the planes may still be read by the sum of the product before
     const int nthr = (kT5Consumers + 1) * 32;
     const int tid = warp < kT5Consumers ? threadIdx.x : kT5Consumers * 32 + lane;
     // one thread places eight consecutive K values of one token: one 16-byte row of a core matrix
@@ -170,7 +173,6 @@ __global__ void __launch_bounds__(kT5Threads, 1) k_gemm_t5(const __grid_constant
     }
     asm volatile("fence.proxy.async.shared::cta;" ::: "memory");   // the tensor core reads xs through the async proxy
   }
-  if (warp < kT5Consumers) table.finish(M.tab32, tab, tab1, warp, lane, kT5Consumers);
   if (warp < kT5Consumers || warp == kT5Consumers + kT5Producers)
     asm volatile("bar.sync 1, %0;" ::"r"((kT5Consumers + 1) * 32) : "memory");
 
