@@ -64,7 +64,7 @@ __global__ void __launch_bounds__(kW16Threads, 1)
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem = tmem_slot[0];
-  // items: splits x tokens x row tiles, row tiles fastest: the blocks that run at one time share a token tile
+  // items: splits x row tiles x token tiles, token tiles fastest: the blocks that read the same rows of W run at one time
   const int items = A.row_tiles * A.tok_tiles * A.splits;
   pdl_trigger();
   if (warp == 0) {
@@ -74,7 +74,7 @@ __global__ void __launch_bounds__(kW16Threads, 1)
       uint32_t ph = 0;
       bool ok = true;
       for (int it = blockIdx.x; it < items && ok; it += gridDim.x) {
-        const int rt = it % A.row_tiles, q = it / A.row_tiles, tt = q % A.tok_tiles, z = q / A.tok_tiles;
+        const int tt = it % A.tok_tiles, q = it / A.tok_tiles, rt = q % A.row_tiles, z = q / A.row_tiles;
         for (int k = 0; k < A.slabs; ++k) {
           if (!(ok = t5_wait(empty + s, ph ^ 1u, A.wait_limit, A.err, abort_flag))) break;
           const uint32_t dst = base + s * stage_bytes;
@@ -125,7 +125,7 @@ __global__ void __launch_bounds__(kW16Threads, 1)
     pdl_wait();   // the factors come from a kernel before, and what it reads may be this kernel's result
     int n = 0;
     for (int it = blockIdx.x; it < items; it += gridDim.x, ++n) {
-      const int rt = it % A.row_tiles, q = it / A.row_tiles, tt = q % A.tok_tiles, z = q / A.tok_tiles;
+      const int tt = it % A.tok_tiles, q = it / A.tok_tiles, rt = q % A.row_tiles, z = q / A.row_tiles;
       const int db = n & 1, row = rt * kW16Rows + quad * 32 + lane, t0 = tt * A.ntok;
       if (!__all_sync(0xffffffffu, t5_wait(d_full + db, (n >> 1) & 1, A.wait_limit, A.err, abort_flag))) break;
       tc_fence_after();
