@@ -2,6 +2,7 @@
 #include <cuda.h>
 
 #include <algorithm>
+#include <cstdlib>
 
 #include "lw_gemv1.h"
 
@@ -21,25 +22,31 @@ int launch_gemm_w16(const __half* X, const __half* W, float* Y, int m, int rows,
   a.tok_tiles = (m + kW16MaxTokens - 1) / kW16MaxTokens;
   a.ntok = ((m + a.tok_tiles - 1) / a.tok_tiles + 15) / 16 * 16;
   a.tok_tiles = (m + a.ntok - 1) / a.ntok;
-  a.row_tiles = (rows + kW16Rows - 1) / kW16Rows;
-  const int slabs = K / kW16SlabK, sms = sm_count(), tiles = a.row_tiles * a.tok_tiles;
-  // Split K where the tiles alone leave blocks idle: the time of a launch is its rounds of work items times an item's
-  // slabs (plus about four slabs' worth of filling and draining), and the planes cost their own traffic: about as long
-  // as 16 slabs for the extra kernel and one per 2 MB written and read again.
-  a.splits = 1;
+  const int slabs = K / kW16SlabK, sms = sm_count();
+  // The tile's rows and the K split, by the time of a launch in ns: rounds of work items times an item's slabs.  A slab takes
+  // what its bytes take at 95 GB/s per SM or its multiply-adds at 1.1 ns per token and 128 rows, whichever is more; filling and
+  // draining about 2 us per launch, and per round where the accumulator is not double-buffered (the tile's results leave
+  // meanwhile: 12 ns per token and 128 rows).  Planes of a split cost the extra kernel, about 4 us, and their own traffic:
+  // 0.35 us per MB.  (Q4_K 14336 x 4096: 256 rows win from 257 tokens on, 128 rows up to 256 tokens.)
+  a.splits = a.blocks_m = 1;
   double best = 0;
-  for (int z = 1; z <= 8; z *= 2) {
-    const size_t plane = static_cast<size_t>(z) * m * rows;
-    if (slabs % z || (z > 1 && (!partials || plane > partial_capacity))) continue;
-    const int rounds = (tiles * z + sms - 1) / sms;
-    const double cost = rounds * (slabs / z + 4.0) + (z > 1 ? 16.0 + plane * 4.0 / (2 << 20) : 0.0);
-    if (z == 1 || cost < best) {
-      best = cost;
-      a.splits = z;
+  for (int b = getenv("LW_B") ? atoi(getenv("LW_B")) : 1; b <= (getenv("LW_B") ? atoi(getenv("LW_B")) : 2); ++b)
+    for (int z = 1; z <= 8; z *= 2) {
+      const size_t plane = static_cast<size_t>(z) * m * rows;
+      if (slabs % z || (z > 1 && (!partials || plane > partial_capacity))) continue;
+      const int tiles = (rows + b * kW16Rows - 1) / (b * kW16Rows) * a.tok_tiles, rounds = (tiles * z + sms - 1) / sms;
+      const double slab = std::max((b * kW16Rows + a.ntok) * 128.0 / 95.0, b * a.ntok * 1.1), out = 2000.0 + b * a.ntok * 12.0;
+      const double cost = rounds * (slabs / z) * slab + (b == 1 ? 1 : rounds) * out + (z > 1 ? 4000.0 + plane * 4.0 / (1 << 20) * 350.0 : 0.0);
+      if (best == 0 || cost < best) {
+        best = cost;
+        a.splits = z;
+        a.blocks_m = b;
+      }
     }
-  }
+  a.row_tiles = (rows + a.blocks_m * kW16Rows - 1) / (a.blocks_m * kW16Rows);
+  const int tiles = a.row_tiles * a.tok_tiles;
   a.slabs = slabs / a.splits;
-  const size_t stage = kW16ABytes + static_cast<size_t>(a.ntok) * kW16SlabK * 2;
+  const size_t stage = a.blocks_m * kW16ABytes + static_cast<size_t>(a.ntok) * kW16SlabK * 2;
   a.stages = static_cast<int>(std::min<size_t>(kW16MaxStages, (kSmemLimit - 2048) / stage));   // 1 KB: the stages' alignment, 1 KB: barriers
   alignas(64) CUtensorMap wm, xm;
   if (!make_half_slab_map(&wm, W, K, rows, kW16Rows) || !make_half_slab_map(&xm, X, K, m, a.ntok)) {
