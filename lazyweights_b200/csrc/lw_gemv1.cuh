@@ -356,9 +356,11 @@ __device__ __forceinline__ void gemv1_block(const MatDev& M, const Gemv1Args& A,
     const size_t src = static_cast<size_t>(set + RA.nsets * j) * TW + k;
     float v[8];
     load_x8(A.x, A.x_is_half, src, v);
-    float amax = 0.f, sum = 0.f;
+    // fmaxf drops a NaN beside a number: starting at a value, not at 0, leaves the maximum (and so the scale and the
+    // product) NaN where a whole sub-block is
+    float amax = fabsf(v[0]), sum = v[0];
 #pragma unroll
-    for (int i = 0; i < 8; ++i) {
+    for (int i = 1; i < 8; ++i) {
       amax = fmaxf(amax, fabsf(v[i]));
       sum += v[i];
     }
