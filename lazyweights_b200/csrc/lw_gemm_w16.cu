@@ -2,7 +2,6 @@
 #include <cuda.h>
 
 #include <algorithm>
-#include <cstdlib>
 
 #include "lw_gemv1.h"
 
@@ -30,7 +29,7 @@ int launch_gemm_w16(const __half* X, const __half* W, float* Y, int m, int rows,
   // 0.35 us per MB.  (Q4_K 14336 x 4096: 256 rows win from 257 tokens on, 128 rows up to 256 tokens.)
   a.splits = a.blocks_m = 1;
   double best = 0;
-  for (int b = getenv("LW_B") ? atoi(getenv("LW_B")) : 1; b <= (getenv("LW_B") ? atoi(getenv("LW_B")) : 2); ++b)
+  for (int b = 1; b <= 2; ++b)
     for (int z = 1; z <= 8; z *= 2) {
       const size_t plane = static_cast<size_t>(z) * m * rows;
       if (slabs % z || (z > 1 && (!partials || plane > partial_capacity))) continue;

@@ -94,3 +94,17 @@ def test_array_addresses_of_the_host_buffer_calls():
     frozen = a.copy()
     frozen.setflags(write=False)
     assert runtime._address(frozen) == frozen.ctypes.data
+
+
+def test_environment_switches_are_documented():
+    """Every variable that the library reads from the environment is in the table of switches: a tuning knob that stays
+    behind in a launcher is an unchecked input of every call."""
+    import glob
+    import os
+    import re
+    root = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
+    table = open(os.path.join(root, "INTEGRATION.md")).read().split("## 5.")[1]
+    read = set()
+    for path in glob.glob(os.path.join(root, "lazyweights_b200", "csrc", "*")):
+        read |= set(re.findall(r'(?:getenv|env_int)\("(LW[A-Z0-9_]*)"', open(path).read()))
+    assert read and not [name for name in sorted(read) if not re.search("`%s[`=]" % name, table)]
