@@ -139,11 +139,13 @@ int lw_matrix_info(void* handle, int id, int* N, int* K, int* fmt, long long* bl
  * of two symbols or, for 11-bit codes under the 10-bit table, to symbol-by-symbol decoding. */
 int lw_matrix_plan(void* handle, int id, int* group, int* index_bits, double* slow_fraction);
 
-/* y[m, N] (fp32, row stride N) = x[m, K] . W^T for 1 <= m <= 8; x is fp16 (x_is_half != 0) or fp32, row-major, on
+/* y[m, N] (fp32, row stride N) = x[m, K] . W^T for m >= 1; x is fp16 (x_is_half != 0) or fp32, row-major, on
  * the device; y_dev must be 16-byte aligned.  Launches on `stream` (a cudaStream_t) and does not synchronise.  This
  * is the device-pointer form of the reference's internal matmul(), kernels/llmrt.cu:1794-1826.  Products of one
  * handle must not overlap on the GPU (they share its split-K scratch, and for m = 1 the matrix's tile-row counters):
- * issue them on one stream, as the reference's runtime does. */
+ * issue them on one stream, as the reference's runtime does.  Up to eight rows nothing is allocated; more rows may
+ * allocate scratch at their first call (one per number of rows that no call before had), so make that call before a
+ * stream capture.  Scratch stays where it is until rt_close: a captured product can be replayed after any other. */
 int lw_linear(void* handle, int id, const void* x_dev, int x_is_half, int m, float* y_dev, void* stream);
 
 /* n one-row products in as few launches as possible: y_j[N_j] = W_j x_j[K_j] for j < n, matrix j = matrix ids[j] of

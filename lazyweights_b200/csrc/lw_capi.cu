@@ -373,6 +373,24 @@ static int grow(T** buf, size_t* have, size_t want, const char* what) {
   return kOk;
 }
 
+// The same for scratch of products that may have been captured: the old buffer stays until the handle is closed, and a
+// buffer at least doubles, so that all those kept are no larger than the one in use.
+template <class T>
+static int grow_kept(Model* M, T** buf, size_t* have, size_t want, const char* what) {
+  if (want <= *have) return kOk;
+  T* bigger = nullptr;
+  size_t n = std::max(want, 2 * *have);
+  if (cudaMalloc(reinterpret_cast<void**>(&bigger), n * sizeof(T)) != cudaSuccess) {   // not twice as much: just enough
+    cudaGetLastError();
+    const cudaError_t e = cudaMalloc(reinterpret_cast<void**>(&bigger), (n = want) * sizeof(T));
+    if (e != cudaSuccess) return cuda_fail(what, e);
+  }
+  if (*buf) M->outgrown.push_back(*buf);
+  *buf = bigger;
+  *have = n;
+  return kOk;
+}
+
 // Activations for the fp16 tensor-core paths: fp16 as they are, fp32 converted with a range factor per row.  *unscale =
 // the factors' inverses (null: none).
 static int half_rows(Model* M, const void* x, bool x_half, int m, int K, const __half** x16, const float** unscale, cudaStream_t st) {
@@ -380,8 +398,8 @@ static int half_rows(Model* M, const void* x, bool x_half, int m, int K, const _
   *unscale = nullptr;
   if (x_half) return kOk;
   int rc;
-  if ((rc = grow(&M->d_x16, &M->x16_halfs, static_cast<size_t>(m) * K, "cudaMalloc (fp16 activations)"))) return rc;
-  if ((rc = grow(&M->d_row_scale, &M->row_scale_floats, static_cast<size_t>(2) * m, "cudaMalloc (row factors)"))) return rc;
+  if ((rc = grow_kept(M, &M->d_x16, &M->x16_halfs, static_cast<size_t>(m) * K, "cudaMalloc (fp16 activations)"))) return rc;
+  if ((rc = grow_kept(M, &M->d_row_scale, &M->row_scale_floats, static_cast<size_t>(2) * m, "cudaMalloc (row factors)"))) return rc;
   if ((rc = launch_rows_to_half(static_cast<const float*>(x), M->d_x16, m, K, M->d_row_scale, st))) return rc;
   *x16 = M->d_x16;
   *unscale = M->d_row_scale + m;
@@ -389,21 +407,28 @@ static int half_rows(Model* M, const void* x, bool x_half, int m, int K, const _
 }
 
 // Decode + GEMM (the reference's path for more than eight rows, kernels/llmrt.cu:1827-1841): tile rows are decoded to
-// fp16 weights in chunks that fit the scratch (grown on first use, at most kDecodeScratchBytes) and multiplied on the
+// fp16 weights in chunks that fit the scratch (allocated on first use for the largest matrix, at most kDecodeScratchBytes) and multiplied on the
 // tensor cores.  128 MB is about the L2 and holds the usual projections whole: a 14336 x 4096 matrix in two chunks of 64 MB cost
 // two launches of each kernel and tiles too few to fill the chip without a K split (32-layer prompt of 128 tokens 11.3 -> 9.9 ms,
 // 512 rows 104 -> 102 us; 256 MB gives the same).
 constexpr size_t kDecodeScratchBytes = size_t(128) << 20;
+static int decode_chunk(const Matrix& mx) {   // tile rows
+  const size_t fit = std::max<size_t>(1, kDecodeScratchBytes / 2 / (static_cast<size_t>(kTileRows) * mx.K));
+  return static_cast<int>(std::min<size_t>(mx.N / kTileRows, fit));
+}
 
 static int linear_decode_gemm(Model* M, Matrix& mx, const __half* x16, const float* unscale, int m, float* y, int ldy,
                               cudaStream_t st) {
   int rc;
   const int NT = mx.N / kTileRows;
   const size_t row_halfs = static_cast<size_t>(kTileRows) * mx.K;
-  const int fit = static_cast<int>(std::max<size_t>(1, kDecodeScratchBytes / 2 / row_halfs));
-  const int chunk = std::min(NT, fit);
-  if ((rc = grow(&M->d_w16, &M->w16_halfs, static_cast<size_t>(chunk) * row_halfs, "cudaMalloc (decoded weights)")))
-    return rc;
+  const int chunk = decode_chunk(mx);
+  if (!M->d_w16) {
+    size_t need = 0;
+    for (const Matrix& m : M->mats)
+      if (m.fmt != kFmtNone) need = std::max(need, static_cast<size_t>(decode_chunk(m)) * kTileRows * m.K);
+    if ((rc = grow_kept(M, &M->d_w16, &M->w16_halfs, need, "cudaMalloc (decoded weights)"))) return rc;
+  }
   for (int tr0 = 0; tr0 < NT; tr0 += chunk) {
     const int tr1 = std::min(NT, tr0 + chunk);
     rc = reads_pairs(mx, 1) ? launch_decode_weights_rows(mx.pair, M->d_w16, tr0, tr1, st) : kErrTooLarge;   // two weights per lookup

@@ -55,10 +55,13 @@ struct Model {
   size_t x_floats = 0, y_floats = 0;
   float* h_pin = nullptr;                 // pinned host staging for the same call (x, then y)
   size_t pin_floats = 0;
+  // Scratch of the products, given to kernels that a caller may have captured into a graph: what is outgrown goes to
+  // `outgrown` and is freed with the handle, so that a replay never touches freed memory.
   __half *d_w16 = nullptr, *d_x16 = nullptr;   // decode + GEMM path: decoded weights of a chunk of tile rows, fp16 x
   size_t w16_halfs = 0, x16_halfs = 0;
   float* d_row_scale = nullptr;   // per-row range factors of fp32 activations headed for fp16 (2 floats per row)
   size_t row_scale_floats = 0;
+  std::vector<void*> outgrown;
   size_t resident_bytes = 0;
   long long coded_bytes = 0, side_bytes = 0;
   Runtime* rt = nullptr;
@@ -76,6 +79,7 @@ struct Model {
     if (d_w16) cudaFree(d_w16);
     if (d_x16) cudaFree(d_x16);
     if (d_row_scale) cudaFree(d_row_scale);
+    for (void* p : outgrown) cudaFree(p);
     if (fd >= 0) close(fd);
   }
 };
