@@ -140,7 +140,7 @@ int lw_matrix_info(void* handle, int id, int* N, int* K, int* fmt, long long* bl
 int lw_matrix_plan(void* handle, int id, int* group, int* index_bits, double* slow_fraction);
 
 /* y[m, N] (fp32, row stride N) = x[m, K] . W^T for m >= 1; x is fp16 (x_is_half != 0) or fp32, row-major, on
- * the device; y_dev must be 16-byte aligned.  Launches on `stream` (a cudaStream_t) and does not synchronise.  This
+ * the device, at any address its type allows; y_dev must be 16-byte aligned.  Launches on `stream` (a cudaStream_t) and does not synchronise.  This
  * is the device-pointer form of the reference's internal matmul(), kernels/llmrt.cu:1794-1826.  Products of one
  * handle must not overlap on the GPU (they share its split-K scratch, and for m = 1 the matrix's tile-row counters):
  * issue them on one stream, as the reference's runtime does.  Up to eight rows nothing is allocated; more rows may

@@ -391,19 +391,20 @@ static int grow_kept(Model* M, T** buf, size_t* have, size_t want, const char* w
   return kOk;
 }
 
-// Activations for the fp16 tensor-core paths: fp16 as they are, fp32 converted with a range factor per row.  *unscale =
-// the factors' inverses (null: none).
+// Activations for the fp16 tensor-core paths, 16-byte aligned: fp16 as they are (copied where the caller's address is not
+// aligned), fp32 converted with a range factor per row.  *unscale = the factors' inverses (null: none).
 static int half_rows(Model* M, const void* x, bool x_half, int m, int K, const __half** x16, const float** unscale, cudaStream_t st) {
   *x16 = static_cast<const __half*>(x);
   *unscale = nullptr;
-  if (x_half) return kOk;
+  if (x_half && !(reinterpret_cast<uintptr_t>(x) & 15u)) return kOk;
   int rc;
-  if ((rc = grow_kept(M, &M->d_x16, &M->x16_halfs, static_cast<size_t>(m) * K, "cudaMalloc (fp16 activations)"))) return rc;
-  if ((rc = grow_kept(M, &M->d_row_scale, &M->row_scale_floats, static_cast<size_t>(2) * m, "cudaMalloc (row factors)"))) return rc;
-  if ((rc = launch_rows_to_half(static_cast<const float*>(x), M->d_x16, m, K, M->d_row_scale, st))) return rc;
+  const size_t count = static_cast<size_t>(m) * K;
+  if ((rc = grow_kept(M, &M->d_x16, &M->x16_halfs, count, "cudaMalloc (fp16 activations)"))) return rc;
   *x16 = M->d_x16;
+  if (x_half) return launch_align_halves(static_cast<const __half*>(x), M->d_x16, count, st);
+  if ((rc = grow_kept(M, &M->d_row_scale, &M->row_scale_floats, static_cast<size_t>(2) * m, "cudaMalloc (row factors)"))) return rc;
   *unscale = M->d_row_scale + m;
-  return kOk;
+  return launch_rows_to_half(static_cast<const float*>(x), M->d_x16, m, K, M->d_row_scale, st);
 }
 
 // Decode + GEMM (the reference's path for more than eight rows, kernels/llmrt.cu:1827-1841): tile rows are decoded to

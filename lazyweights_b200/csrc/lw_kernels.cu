@@ -232,6 +232,20 @@ __global__ void __launch_bounds__(kToHalfThreads)
   for (int k = kToHalfHeld * kToHalfThreads + threadIdx.x; k < quads; k += kToHalfThreads) out[k] = halves(load(k));
 }
 
+// Halves at any even address -> the same at a 16-byte aligned one (n pieces of eight): the tensor-core kernels read their
+// activations with 16-byte loads and tile copies.
+__global__ void __launch_bounds__(256) k_align_halves(const __half* src, uint4* dst, int n) {
+  pdl_trigger();
+  pdl_wait();
+  const int i = blockIdx.x * 256 + threadIdx.x;
+  if (i >= n) return;
+  const unsigned short* s = reinterpret_cast<const unsigned short*>(src) + static_cast<size_t>(i) * 8;
+  uint32_t w[4];
+#pragma unroll
+  for (int j = 0; j < 4; ++j) w[j] = s[2 * j] | static_cast<uint32_t>(s[2 * j + 1]) << 16;
+  dst[i] = make_uint4(w[0], w[1], w[2], w[3]);
+}
+
 // Y[j, n] = sum over the `terms` partial rows of P[term, j, n], in a fixed order (no atomics: results do not depend on
 // scheduling).  Four consecutive outputs per thread, PARTS threads per four outputs: part p adds terms p, p + PARTS, ...,
 // then the parts are added with shuffles.  What bounds it is the chain of round trips to L2, one per eight terms of a thread:
@@ -668,6 +682,12 @@ int launch_pull(const void* host_src, void* dst, size_t bytes, cudaStream_t st) 
 int launch_rows_to_half(const float* src, __half* dst, int m, int K, float* scales, cudaStream_t st) {
   launch_dependent(k_rows_to_half, dim3(m), dim3(kToHalfThreads), st, src, dst, K, m, scales);
   return check_launch("k_rows_to_half");
+}
+
+int launch_align_halves(const __half* src, __half* dst, size_t count, cudaStream_t st) {
+  const int n = static_cast<int>(count / 8);
+  launch_dependent(k_align_halves, dim3((n + 255) / 256), dim3(256), st, src, reinterpret_cast<uint4*>(dst), n);
+  return check_launch("k_align_halves");
 }
 
 int launch_sum_partials(const float* P, float* Y, int m, int N, int ldy, int terms, const float* unscale, cudaStream_t st) {

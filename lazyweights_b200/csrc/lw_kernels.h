@@ -51,8 +51,10 @@ int launch_pull(const void* host_src, void* dst, size_t bytes, cudaStream_t st);
 // inside fp16's range (1 unless the row holds values above 2^15), scales[m + r] = its inverse, to be applied to row r of
 // the product.
 int launch_rows_to_half(const float* src, __half* dst, int m, int K, float* scales, cudaStream_t st);
+// dst (16-byte aligned) = `count` halves (a multiple of eight) at any address.
+int launch_align_halves(const __half* src, __half* dst, size_t count, cudaStream_t st);
 // Y[m, rows] (row stride ldy) = X[m, K] . W[rows, K]^T for the decode + GEMM path: fp16 in, fp32 out, tensor cores.
-// unscale (may be null): factor per row of X, applied to the finished sums.
+// unscale (may be null): factor per row of X, applied to the finished sums.  X: 16-byte aligned.
 int launch_gemm_w16(const __half* X, const __half* W, float* Y, int m, int rows, int K, int ldy, float* partials,
                     size_t partial_capacity, const float* unscale, cudaStream_t st);
 // Y[j, n] (row stride ldy) = sum_k X[j, k] W[n, k] for m <= 8 rows of X (fp16 or fp32, row-major [m, K]).
@@ -64,7 +66,7 @@ int launch_gemv(const MatDev& M, const void* X, bool x_is_half, int m, float* Y,
                 size_t partial_capacity, cudaStream_t st, unsigned int* clean_epoch = nullptr);
 // Y[m, N] = X[m, K] . W^T for 1 <= m <= 64 with the decode + tcgen05 kernel (lw_gemm_t5.cuh): the decoded weights go
 // from registers to tensor memory, never to DRAM.  `scratch` holds the K / 512 planes of partial products.  Returns
-// kErrTooLarge, with nothing launched, where that kernel cannot take the product.  unscale: as in launch_gemm_w16.
+// kErrTooLarge, with nothing launched, where that kernel cannot take the product.  X, unscale: as in launch_gemm_w16.
 int launch_gemm_coded(const MatDev& M, const __half* X, const float* unscale, int m, float* Y, int ldy, float* scratch,
                       size_t scratch_floats, cudaStream_t st);
 

@@ -68,3 +68,20 @@ def test_q5k_pair_code_lengths(lw, n, k, wide):
             x = rng.standard_normal((m, k)).astype(np.float32)
             y = mat.linear("m", torch.from_numpy(x).cuda()).cpu().numpy()
             assert helpers.rel_err(y, orc.gemv_f64(w, x)) <= TOL, m
+
+
+# Activations at an address that only their own type allows: every kernel has its wide loads, every row count its kernel
+@pytest.mark.parametrize("ty,n,k", [("Q4_K", 256, 1024), ("Q6_K", 256, 1536), ("Q5_K", 192, 256)])
+@pytest.mark.parametrize("half", [True, False])
+def test_unaligned_activations(lw, ty, n, k, half):
+    import torch
+    q, side, sym, w, rng = helpers.seeded_case(ty, n, k, seed=n + 5 * k)
+    blob, _, _ = lw.bundle.encode_huf8(sym)
+    with lw.CodedMatrix(blob, n, sym.shape[1], ty, side) as mat:
+        for m in (1, 2, 8, 9, 16, 33, 64, 65, 300):
+            x = torch.from_numpy(rng.standard_normal((m, k)).astype(np.float16 if half else np.float32)).cuda()
+            want = mat.linear("m", x)
+            for off in (1, 2):
+                z = torch.empty(m * k + off, dtype=x.dtype, device="cuda")
+                z[off:] = x.reshape(-1)
+                assert torch.equal(mat.linear("m", z[off:].reshape(m, k)), want), (m, off)
