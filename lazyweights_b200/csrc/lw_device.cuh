@@ -57,7 +57,10 @@ __device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity, unsigne
 // Programmatic dependent launch: a kernel launched with the stream-serialization attribute may start while its
 // predecessor in the stream is still running (as soon as every block of the predecessor has called pdl_trigger or
 // left), and must call pdl_wait before it touches anything the predecessor writes: the wait returns when the
-// predecessor has completed and its writes are visible.  Without the launch attribute both are no-ops.
+// predecessor has completed and its writes are visible.  Without the launch attribute both are no-ops.  What the
+// predecessor writes is not read-only while such a kernel lives, so it is not read with __ldg or through const
+// __restrict__ pointers (the read-only path may answer from a line that it fetched before, and such a load may be moved
+// over the wait): ordinary loads.
 __device__ __forceinline__ void pdl_trigger() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 __device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 

@@ -180,7 +180,7 @@ __global__ void __launch_bounds__(kWarpsPerBlock * 32)
 // for the maxima and 4 us for the conversion as two kernels of scalar loads.
 constexpr int kToHalfThreads = 512, kToHalfHeld = 8;
 __global__ void __launch_bounds__(kToHalfThreads)
-    k_rows_to_half(const float* __restrict__ src, __half* __restrict__ dst, int K, int m, float* __restrict__ scales) {
+    k_rows_to_half(const float* src, __half* __restrict__ dst, int K, int m, float* __restrict__ scales) {
   __shared__ float part[kToHalfThreads / 32];
   pdl_trigger();
   pdl_wait();
@@ -253,8 +253,8 @@ __global__ void __launch_bounds__(256) k_align_halves(const __half* src, uint4* 
 // (now about 5 and 4: a 32-layer pass of eight tokens 5.49 -> 4.30 ms; Q6_K 14336 x 4096, eight rows, 49.6 -> 40.5 us).
 // unscale (may be null): factor per output row j, applied to the finished sum.
 template <int PARTS>
-__global__ void __launch_bounds__(128) k_sum_partials(const float* __restrict__ P, float* __restrict__ Y, int m, int N, int ldy, int terms,
-                                                      const float* __restrict__ unscale) {
+__global__ void __launch_bounds__(128) k_sum_partials(const float* P, float* __restrict__ Y, int m, int N, int ldy, int terms,
+                                                      const float* unscale) {
   pdl_trigger();   // launched as a programmatic dependent of the kernel that writes P (see lw_device.cuh)
   pdl_wait();
   constexpr int QW = 32 / PARTS;   // groups of four outputs per warp: neighbouring lanes, so that a part's loads are contiguous
@@ -268,7 +268,7 @@ __global__ void __launch_bounds__(128) k_sum_partials(const float* __restrict__ 
   for (int t0 = part; t0 < terms; t0 += 8 * PARTS) {
     float4 v[8];
 #pragma unroll
-    for (int u = 0; u < 8; ++u) v[u] = t0 + u * PARTS < terms ? __ldg(p + (t0 + u * PARTS) * stride) : make_float4(0.f, 0.f, 0.f, 0.f);
+    for (int u = 0; u < 8; ++u) v[u] = t0 + u * PARTS < terms ? p[(t0 + u * PARTS) * stride] : make_float4(0.f, 0.f, 0.f, 0.f);
 #pragma unroll
     for (int u = 0; u < 8; ++u) {
       acc.x += v[u].x;

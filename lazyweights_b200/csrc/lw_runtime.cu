@@ -126,7 +126,9 @@ __global__ void k_embed8(const int* __restrict__ ids, const uint8_t* __restrict_
 }
 
 // Programmatic dependent launch (see lw_device.cuh): every kernel of a pass lets its successor be set up at once and
-// waits for its predecessor before it reads or writes anything.
+// waits for its predecessor before it reads or writes anything.  Such a kernel is resident while the predecessor still
+// writes, so what the predecessor wrote is not read-only for the kernel's lifetime: it is read with ordinary loads through
+// pointers that are not const __restrict__, never with __ldg.
 __device__ __forceinline__ void dep_begin() {
   asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
   asm volatile("griddepcontrol.wait;" ::: "memory");
@@ -150,7 +152,7 @@ static void launch_dep(void (*kernel)(KArgs...), dim3 grid, dim3 block, cudaStre
 // to eight elements in registers (float4 loads), so the row is read once.  Longer rows fall back to a second read.
 constexpr int kNormThreads = 1024;
 __global__ void __launch_bounds__(kNormThreads)
-    k_rmsnorm(float* __restrict__ h, const float* __restrict__ res, const float* __restrict__ g,
+    k_rmsnorm(float* __restrict__ h, const float* res, const float* __restrict__ g,
               float* __restrict__ out, int D, float eps) {
   dep_begin();
   __shared__ float red[33];
@@ -239,7 +241,7 @@ __host__ __device__ constexpr size_t peer_flag_words() { return 2 * kPeerMaxBloc
 __host__ __device__ inline size_t peer_slot_floats(int D) { return static_cast<size_t>(2) * kPeerMaxRanks * kPeerMaxBlocks * D; }
 
 __global__ void __launch_bounds__(kNormThreads)
-    k_allreduce_rmsnorm(PeerView P, const float* __restrict__ part, float* __restrict__ h, const float* __restrict__ g,
+    k_allreduce_rmsnorm(PeerView P, const float* part, float* __restrict__ h, const float* __restrict__ g,
                         float* __restrict__ out, float eps, unsigned int* err, uint32_t limit) {
   dep_begin();
   __shared__ float red[33];
@@ -315,7 +317,7 @@ __global__ void __launch_bounds__(kNormThreads)
 
 // rotate-half RoPE on q (in place) and k (into the cache), v into the cache.  grid (heads + 2 kv heads, tokens).
 __global__ void k_rope_cache(float* __restrict__ qkv, const float* __restrict__ cosv, const float* __restrict__ sinv,
-                             __half* __restrict__ kc, __half* __restrict__ vc, const int* __restrict__ posp, int H, int Hk,
+                             __half* __restrict__ kc, __half* __restrict__ vc, const int* posp, int H, int Hk,
                              int Dh, int Tmax) {
   dep_begin();
   const int head = blockIdx.x, j = blockIdx.y, p = *posp + j, half = Dh / 2;
@@ -355,9 +357,9 @@ constexpr int kAttnStride = kAttnMaxDh / 2 + 1;   // words per staged row: odd, 
 // staged once in shared memory (16-byte loads) and serve all of them.
 template <int GH>
 __global__ void __launch_bounds__(kAttnThreads)
-    k_attn(const float* __restrict__ qkv, const __half* __restrict__ kc, const __half* __restrict__ vc,
+    k_attn(const float* qkv, const __half* kc, const __half* vc,
            float* __restrict__ part, float* __restrict__ att, unsigned int* __restrict__ done,
-           const int* __restrict__ posp, int H, int Hk, int Dh, int Tmax, float scale, int window, int max_chunks) {
+           const int* posp, int H, int Hk, int Dh, int Tmax, float scale, int window, int max_chunks) {
   dep_begin();
   __shared__ uint32_t kv[kAttnChunk * kAttnStride];
   __shared__ float qs[GH][kAttnMaxDh];
@@ -385,7 +387,7 @@ __global__ void __launch_bounds__(kAttnThreads)
       for (int idx = threadIdx.x; idx < kAttnChunk * cpr; idx += kAttnThreads) {
         const int t = idx / cpr, ch = idx - t * cpr;
         uint4 v = make_uint4(0u, 0u, 0u, 0u);
-        if (t < n) v = __ldg(reinterpret_cast<const uint4*>(src + static_cast<size_t>(t) * Dh) + ch);
+        if (t < n) v = reinterpret_cast<const uint4*>(src + static_cast<size_t>(t) * Dh)[ch];
         uint32_t* d = kv + t * kAttnStride + ch * 4;
         d[0] = v.x;
         d[1] = v.y;
@@ -404,7 +406,7 @@ __global__ void __launch_bounds__(kAttnThreads)
       for (int u = 0; u < VPT; ++u) {
         const int idx = threadIdx.x + u * kAttnThreads, t = idx / cpr, ch = idx - t * cpr;
         vreg[u] = make_uint4(0u, 0u, 0u, 0u);
-        if (idx < kAttnChunk * cpr && t < n) vreg[u] = __ldg(reinterpret_cast<const uint4*>(vsrc + static_cast<size_t>(t) * Dh) + ch);
+        if (idx < kAttnChunk * cpr && t < n) vreg[u] = reinterpret_cast<const uint4*>(vsrc + static_cast<size_t>(t) * Dh)[ch];
       }
     }
     __syncthreads();
@@ -579,9 +581,9 @@ constexpr int kRowsMaxSpans = 32;                  // a lane of the merge holds 
 
 template <int RW>
 __global__ void __launch_bounds__(kAttnThreads, 2)
-    k_attn_rows(const float* __restrict__ qkv, const __half* __restrict__ kc, const __half* __restrict__ vc,
+    k_attn_rows(const float* qkv, const __half* kc, const __half* vc,
                 float* __restrict__ part, float* __restrict__ att, unsigned int* __restrict__ done,
-                const int* __restrict__ posp, int m, int H, int Hk, int Dh, int Tmax, float scale, int window, int max_chunks) {
+                const int* posp, int m, int H, int Hk, int Dh, int Tmax, float scale, int window, int max_chunks) {
   dep_begin();
   constexpr int R = kAttnThreads / 32 * RW;
   __shared__ __align__(16) uint32_t kv[kAttnChunk * kRowsStride];
@@ -623,7 +625,7 @@ __global__ void __launch_bounds__(kAttnThreads, 2)
     for (int u = 0; u < VPT; ++u) {
       const int idx = threadIdx.x + u * kAttnThreads, t = idx / cpr, ch = idx - t * cpr;
       reg[u] = make_uint4(0u, 0u, 0u, 0u);
-      if (idx < kAttnChunk * cpr && t < n) reg[u] = __ldg(reinterpret_cast<const uint4*>(src + static_cast<size_t>(t) * Dh) + ch);
+      if (idx < kAttnChunk * cpr && t < n) reg[u] = reinterpret_cast<const uint4*>(src + static_cast<size_t>(t) * Dh)[ch];
     }
   };
   auto place = [&](const uint4 (&reg)[VPT]) {
@@ -812,7 +814,7 @@ __global__ void __launch_bounds__(kAttnThreads, 2)
 // with W ranks the rank-major gather of their slices (slot r: Vmax floats, the first (base + (r < rem)) * 64 valid, ids
 // from (r * base + min(r, rem)) * 64).  ids[0] = token of the next pass, ids[B] = its position, ids[B + 1] = tokens
 // generated so far.  One block.
-__global__ void __launch_bounds__(1024) k_argmax_next(const float* __restrict__ logits, int W, int Vmax, int base, int rem,
+__global__ void __launch_bounds__(1024) k_argmax_next(const float* logits, int W, int Vmax, int base, int rem,
                                                       int* __restrict__ ids, int B, int* __restrict__ gen) {
   dep_begin();
   __shared__ float sv[32];
@@ -873,7 +875,7 @@ __global__ void __launch_bounds__(1024) k_argmax_next(const float* __restrict__ 
   }
 }
 
-__global__ void k_silu_mul(float* __restrict__ g, const float* __restrict__ u, size_t n) {
+__global__ void k_silu_mul(float* __restrict__ g, const float* u, size_t n) {
   dep_begin();
   const size_t i = blockIdx.x * static_cast<size_t>(blockDim.x) + threadIdx.x;
   if (i < n) {

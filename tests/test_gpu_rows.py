@@ -85,3 +85,21 @@ def test_unaligned_activations(lw, ty, n, k, half):
                 z = torch.empty(m * k + off, dtype=x.dtype, device="cuda")
                 z[off:] = x.reshape(-1)
                 assert torch.equal(mat.linear("m", z[off:].reshape(m, k)), want), (m, off)
+
+
+def test_scratch_reused_back_to_back(lw):
+    """Products in a row on one handle write and read the same scratch, each kernel set up while the one before still
+    runs: every result is the one that the product gives alone."""
+    import torch
+    q, side, sym, w, rng = helpers.seeded_case("Q4_K", 512, 2048, seed=77)
+    blob, _, _ = lw.bundle.encode_huf8(sym)
+    with lw.CodedMatrix(blob, 512, sym.shape[1], "Q4_K", side) as mat:
+        xs = [torch.from_numpy(rng.standard_normal((m, 2048)).astype(np.float32)).cuda() for m in (8, 9, 33, 33, 64, 80, 80, 200)]
+        want = []
+        for x in xs:
+            want.append(mat.linear("m", x).clone())
+            torch.cuda.synchronize()
+        order = rng.integers(0, len(xs), 300)
+        got = [mat.linear("m", xs[i]) for i in order]
+        for i, y in zip(order, got):
+            assert torch.equal(y, want[i])
