@@ -299,7 +299,8 @@ long long lw_launch_count(void);
  * "wait_limit" (polls after which a device-side wait gives up), "drop_unit" (block 0's producers never copy this unit
  * of their list, so the waits for it run out; -1 = none), "t5_min_rows" (1..65: products of at least this many rows,
  * and at most 64, take the decode + tcgen05 kernel; 9 in production), "pairs" (0 / 1: product kernels read the bundle's own code even
- * where a matrix has a pair layout), "reset" (all back to the production values). */
+ * where a matrix has a pair layout), "attn_rows" (0: passes of several tokens take the attention kernel with a block per token, not
+ * the tiled one; passes captured before keep theirs), "reset" (all back to the production values). */
 int lw_debug_set(const char* key, long long value);
 /* Test hook for the bounded wait above: holds the handle's stream up with a host function that sleeps `ms`
  * milliseconds (0..5000; the GPU is idle meanwhile) and runs the bounded wait with the handle's timeout: 0 if the

@@ -531,6 +531,7 @@ int lw_debug_set(const char* key, long long value) {
   else if (s == "drop_unit" && value >= -1 && value < 1024) k.drop_unit = static_cast<int>(value);
   else if (s == "t5_min_rows" && value >= 1 && value <= 65) k.t5_min_rows = static_cast<int>(value);
   else if (s == "pairs" && (value == 0 || value == 1)) k.pairs = static_cast<int>(value);
+  else if (s == "attn_rows" && (value == 0 || value == 1)) k.attn_rows = static_cast<int>(value);
   else if (s == "reset") k = DebugKnobs();
   else {
     set_error("lw_debug_set: unknown key or value out of range (%s)", key);

@@ -43,6 +43,7 @@ struct DebugKnobs {
   int t5_min_rows = 9;             // products of at least this many rows (and at most 64) take the tcgen05 kernel (eight
                                    // rows: the fused kernel, 46-49 against 54 us on 14336 x 4096 in all four formats)
   int pairs = 1;                   // one-row products read a matrix's pair layout where it has one (0: the bundle's code)
+  int attn_rows = 1;               // passes of several tokens take the tiled attention (0: k_attn, a block per token)
 };
 DebugKnobs& debug_knobs();
 

@@ -347,11 +347,79 @@ __global__ void k_rope_cache(float* __restrict__ qkv, const float* __restrict__ 
 // score maximum, its sum of exponentials and the unnormalised weighted sum of v; the block that finishes LAST for a
 // (head group, token) merges the chunks with the usual running-maximum rescaling (a counter per (token, head group)
 // that the last block sets back to zero), so no second kernel and no wait: every block but one just leaves.  Per-query
-// arithmetic does not depend on how many tokens the pass carries, nor on which block happens to be last (the merge
-// always runs over the chunks in order).  Chunks of 64 positions: 256 blocks for a context of 2048 and 8 kv heads
+// arithmetic does not depend on how many tokens the pass carries (nor on k_attn_rows serving it), nor on which block happens
+// to be last (the merge always runs over the chunks in order).  Chunks of 64 positions: 256 blocks for a context of 2048 and 8 kv heads
 // (with 128 positions and a separate merge kernel attention took 0.51 of 3.51 ms per token of the 7B-shaped model).
 constexpr int kAttnChunk = 64, kAttnThreads = 256, kAttnMaxDh = 128;
 constexpr int kAttnStride = kAttnMaxDh / 2 + 1;   // words per staged row: odd, so 32 consecutive rows hit 32 banks
+
+// The merge of RW query rows by one warp: at base + i * row_stride are row i's chunks, Dh + 2 floats each (maximum, sum of
+// exponentials, weighted sum of v), n[i] of them; res[i] = dimensions 4 lane .. 4 lane + 3 of row i.  Every row is merged
+// the same way whatever RW is: the total by lanes that hold every 32nd chunk, the outputs chunk after chunk.  EMPTY: a
+// chunk may hold nothing - its sum is 0 and its vector was not written; without it the vectors' loads need not wait for the sums.
+template <int RW, bool EMPTY>
+__device__ __forceinline__ void merge_chunks(const float* base, size_t row_stride, const int (&n)[RW], int Dh, int lane, float4 (&res)[RW]) {
+  const int stride = Dh + 2;
+  const bool mine = lane * 4 < Dh;
+  auto head = [&](int i, int c) {
+    return c < n[i] ? __ldcg(reinterpret_cast<const float2*>(base + i * row_stride + static_cast<size_t>(c) * stride)) : make_float2(-INFINITY, 0.f);
+  };
+  float2 ms[RW];
+  float top[RW], tot[RW];
+  int longest = 0;
+#pragma unroll
+  for (int i = 0; i < RW; ++i) ms[i] = head(i, lane);
+#pragma unroll
+  for (int i = 0; i < RW; ++i) {
+    longest = max(longest, n[i]);
+    top[i] = ms[i].x;
+    for (int c = lane + 32; c < n[i]; c += 32) top[i] = fmaxf(top[i], head(i, c).x);
+    for (int o = 16; o; o >>= 1) top[i] = fmaxf(top[i], __shfl_xor_sync(0xffffffffu, top[i], o));
+    tot[i] = 0.f;
+    res[i] = make_float4(0.f, 0.f, 0.f, 0.f);
+  }
+  for (int cb = 0; cb < longest; cb += 32) {
+    float w[RW];
+    uint32_t held[RW];
+#pragma unroll
+    for (int i = 0; i < RW; ++i) {
+      if (cb) ms[i] = head(i, cb + lane);
+      w[i] = ms[i].y > 0.f ? __expf(ms[i].x - top[i]) : 0.f;
+      tot[i] += ms[i].y * w[i];
+      held[i] = EMPTY ? __ballot_sync(0xffffffffu, ms[i].y != 0.f) : 0xffffffffu;
+    }
+    constexpr int U = RW == 4 ? 2 : 16 / RW;   // chunks whose vectors are in flight
+    for (int z0 = 0; z0 < 32 && cb + z0 < longest; z0 += U) {
+      float2 x[RW][U], y[RW][U];
+#pragma unroll
+      for (int i = 0; i < RW; ++i)
+#pragma unroll
+        for (int u = 0; u < U; ++u) {
+          x[i][u] = y[i][u] = make_float2(0.f, 0.f);
+          if (cb + z0 + u < n[i] && (!EMPTY || (held[i] >> (z0 + u) & 1u)) && mine) {
+            const float2* p = reinterpret_cast<const float2*>(base + i * row_stride + static_cast<size_t>(cb + z0 + u) * stride);
+            x[i][u] = __ldcg(p + 1 + 2 * lane);
+            y[i][u] = __ldcg(p + 2 + 2 * lane);
+          }
+        }
+#pragma unroll
+      for (int i = 0; i < RW; ++i)
+#pragma unroll
+        for (int u = 0; u < U; ++u) {   // in chunk order
+          const float wz = __shfl_sync(0xffffffffu, w[i], z0 + u);
+          res[i].x = fmaf(wz, x[i][u].x, res[i].x);
+          res[i].y = fmaf(wz, x[i][u].y, res[i].y);
+          res[i].z = fmaf(wz, y[i][u].x, res[i].z);
+          res[i].w = fmaf(wz, y[i][u].y, res[i].w);
+        }
+    }
+  }
+#pragma unroll
+  for (int i = 0; i < RW; ++i) {
+    for (int o = 16; o; o >>= 1) tot[i] += __shfl_xor_sync(0xffffffffu, tot[i], o);
+    res[i] = make_float4(res[i].x / tot[i], res[i].y / tot[i], res[i].z / tot[i], res[i].w / tot[i]);
+  }
+}
 
 // GH query heads that share one kv head (grouped-query attention) per block: the chunk's keys, then its values, are
 // staged once in shared memory (16-byte loads) and serve all of them.
@@ -536,7 +604,8 @@ __global__ void __launch_bounds__(kAttnThreads)
       for (int c0 = 0; c0 < nchunks; c0 += 16) {
         float v[16];
 #pragma unroll
-        for (int u = 0; u < 16; ++u) v[u] = c0 + u < nchunks ? __ldcg(col + static_cast<size_t>(c0 + u) * (Dh + 2)) : 0.f;
+        for (int u = 0; u < 16; ++u)   // an empty chunk's vector was not written
+          v[u] = c0 + u < nchunks && sums[h * nchunks + c0 + u] != 0.f ? __ldcg(col + static_cast<size_t>(c0 + u) * (Dh + 2)) : 0.f;
 #pragma unroll
         for (int u = 0; u < 16; ++u) a = fmaf(c0 + u < nchunks ? w[c0 + u] : 0.f, v[u], a);   // in chunk order
       }
@@ -544,46 +613,41 @@ __global__ void __launch_bounds__(kAttnThreads)
     }
     return;
   }
-  for (int o = threadIdx.x; o < GH * Dh; o += kAttnThreads) {   // very long contexts: chunk by chunk
-    const int h = o / Dh, d = o - h * Dh;
-    float mx = -INFINITY;
-    for (int ch = 0; ch < nchunks; ++ch) mx = fmaxf(mx, __ldcg(out_of(h, ch)));
-    float tot = 0.f, a = 0.f;
-    for (int ch = 0; ch < nchunks; ++ch) {
-      const float* pc = out_of(h, ch);
-      const float sum = __ldcg(pc + 1);
-      if (sum > 0.f) {
-        const float w = __expf(__ldcg(pc) - mx);
-        tot += sum * w;
-        a += __ldcg(pc + 2 + d) * w;
-      }
-    }
-    att[static_cast<size_t>(j) * H * Dh + static_cast<size_t>(head0 + h) * Dh + d] = a / tot;
+  if (warp < GH) {   // very long contexts: a warp per head, the same sums in the same order
+    const int n1[1] = {nchunks};
+    float4 res[1];
+    merge_chunks<1, true>(out_of(warp, 0), 0, n1, Dh, lane, res);
+    if (lane * 4 < Dh) *reinterpret_cast<float4*>(att + static_cast<size_t>(j) * H * Dh + static_cast<size_t>(head0 + warp) * Dh + lane * 4) = res[0];
   }
 }
 
-// The same attention for passes of several tokens.  A block of k_attn serves one token, so a pass of m tokens read every key
-// and value m times and staged them m times: 252 us for 64 tokens at a context of 2048 (8 kv heads, 4 query heads each),
-// 48.7 us for 8 tokens at 1008 (32 kv heads).  Here a block serves a tile of R = 8 RW query rows of one kv head - row r of the
-// pass is head r % group of token r / group - so a chunk is read once per tile; bound: fp32 multiply-adds from about 16 rows
-// on, below that the latency of the chunks' loads.
-//  * A warp owns RW rows for the whole kernel: its scores, running maximum, sum and outputs stay in registers, and nothing
-//    but the staged chunk is shared between warps.  Lane l holds the scores of positions l and l + 32 of the chunk and, in
-//    the value phase, dimensions 4 l .. 4 l + 3.  Per eight dimensions a warp reads 16 wavefronts of keys and queries for
-//    64 RW / 4 multiply-adds: at RW = 4 both pipes are equally busy.
-//  * A block walks a span of chunks with the running-maximum rescaling.  While it works on keys the values of the chunk are on
-//    their way into registers, while it works on values the next chunk's keys are.
-//  * Spans: as many per tile as bring two blocks to every SM; their results are merged in span order by the block that is last
-//    (the counter of k_attn).  Chunks per span follow from the position on the device, so a captured pass covers any of its bucket.
+// The same attention for passes of several tokens whose ranges all start at position 0 (no window, or one that is not yet
+// full).  A block of k_attn serves one token, so a pass of m tokens reads every key and value m times and stages them m
+// times: 252 us for 64 tokens at a context of 2048 (8 kv heads, 4 query heads each), 48.7 us for 8 tokens at 1008 (32 kv
+// heads).  Here a block serves a tile of R = 8 RW query rows of one kv head - row r of the pass is head r % group of token
+// r / group - so a chunk is read once per tile; bound: fp32 multiply-adds from about 16 rows on, below that the latency of
+// the chunks' loads.
+//  * A warp owns RW rows for the whole kernel, so nothing but the staged chunk is shared between warps.  Lane l holds the
+//    scores of positions l and l + 32 of the chunk and, in the value phase, dimensions 4 l .. 4 l + 3.  Per eight
+//    dimensions a warp reads 16 wavefronts of keys and queries for 64 RW / 4 multiply-adds: at RW = 4 both pipes are
+//    equally busy.
+//  * A block walks a span of chunks.  While it works on keys the values of the chunk are on their way into registers, while
+//    it works on values the next chunk's keys are.
+//  * The arithmetic is k_attn's, bit for bit: the same chunks of 64 positions, every sum in the same order, and each
+//    chunk's maximum, sum and outputs kept apart until all are merged in chunk order.  How many tokens a pass carries, and so
+//    how its rows fall into tiles and its chunks into spans, leaves a query's result alone.  (Rescaling along a span instead of
+//    keeping its chunks apart would save their way through L2: 1 of 134 us per layer of an 8-token pass at 1000 positions
+//    with 32 kv heads, 13 of 140 at 4000 positions with 8.)
+//  * Spans: as many per tile as bring two blocks to every SM; the block that is last (the counter of k_attn) merges.  Chunks
+//    per span follow from the position on the device, so a captured pass covers any of its bucket.
 // Queries, scores, probabilities and sums are fp32, as in k_attn.
 constexpr int kRowsStride = kAttnMaxDh / 2 + 4;   // words per staged row: 16-byte aligned, 8 lanes' 16-byte loads hit 32 banks
-constexpr int kRowsMaxSpans = 32;                  // a lane of the merge holds one span
 
 template <int RW>
 __global__ void __launch_bounds__(kAttnThreads, 2)
     k_attn_rows(const float* qkv, const __half* kc, const __half* vc,
                 float* __restrict__ part, float* __restrict__ att, unsigned int* __restrict__ done,
-                const int* posp, int m, int H, int Hk, int Dh, int Tmax, float scale, int window, int max_chunks) {
+                const int* posp, int m, int H, int Hk, int Dh, int Tmax, float scale, int max_chunks) {
   dep_begin();
   constexpr int R = kAttnThreads / 32 * RW;
   __shared__ __align__(16) uint32_t kv[kAttnChunk * kRowsStride];
@@ -592,22 +656,16 @@ __global__ void __launch_bounds__(kAttnThreads, 2)
   __shared__ unsigned int s_last;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int group = H / Hk, rows = m * group, kh = blockIdx.x, r0 = blockIdx.y * R, spans = gridDim.z, pos = *posp;
-  const int t_first = r0 / group, t_last = (min(rows, r0 + R) - 1) / group;
-  const int hi = pos + t_last + 1, lo = window > 0 ? max(0, pos + t_first - window + 1) : 0;   // positions any row of the tile sees
-  const int total = (hi - lo + kAttnChunk - 1) / kAttnChunk, per = (total + spans - 1) / spans;
+  const int hi = pos + (min(rows, r0 + R) - 1) / group + 1;   // positions any row of the tile sees
+  const int total = (hi + kAttnChunk - 1) / kAttnChunk, per = (total + spans - 1) / spans;
   const int c0 = blockIdx.z * per, c1 = min(total, c0 + per);
-  // this warp's rows: token, head, first and last position they see (rows past the end see nothing)
+  // this warp's rows: the last position they see (rows past the end see nothing)
   const int row0 = r0 + warp * RW;
-  int first[RW], last[RW], all_first = 0, all_last = 0x7fffffff;
+  int last[RW], all_last = 0x7fffffff;
 #pragma unroll
   for (int i = 0; i < RW; ++i) {
-    const int t = (row0 + i) / group;
-    last[i] = row0 + i < rows ? pos + t : -1;
-    first[i] = window > 0 ? max(0, pos + t - window + 1) : 0;
-    if (row0 + i < rows) {
-      all_first = max(all_first, first[i]);
-      all_last = min(all_last, last[i]);
-    }
+    last[i] = row0 + i < rows ? pos + (row0 + i) / group : -1;
+    if (row0 + i < rows) all_last = min(all_last, last[i]);
   }
   for (int i = threadIdx.x; i < R * (Dh / 4); i += kAttnThreads) {
     const int r = i / (Dh / 4), d = (i - r * (Dh / 4)) * 4, g = r0 + r;
@@ -619,7 +677,7 @@ __global__ void __launch_bounds__(kAttnThreads, 2)
   const int cpr = Dh / 8;                                              // 16-byte pieces per row
   constexpr int VPT = kAttnChunk * (kAttnMaxDh / 8) / kAttnThreads;    // pieces per thread (4)
   auto fetch = [&](const __half* base, int c, uint4 (&reg)[VPT]) {
-    const int p0 = lo + c * kAttnChunk, n = min(kAttnChunk, hi - p0);
+    const int p0 = c * kAttnChunk, n = min(kAttnChunk, hi - p0);
     const __half* src = base + (static_cast<size_t>(kh) * Tmax + p0) * Dh;
 #pragma unroll
     for (int u = 0; u < VPT; ++u) {
@@ -635,14 +693,11 @@ __global__ void __launch_bounds__(kAttnThreads, 2)
       if (idx < kAttnChunk * cpr) *reinterpret_cast<uint4*>(kv + t * kRowsStride + ch * 4) = reg[u];
     }
   };
-  float mx[RW], sum[RW], out[RW][4];
-#pragma unroll
-  for (int i = 0; i < RW; ++i) {
-    mx[i] = -INFINITY;
-    sum[i] = 0.f;
-#pragma unroll
-    for (int d = 0; d < 4; ++d) out[i][d] = 0.f;
-  }
+  auto chunk_of = [&](int i, int c) { return part + ((static_cast<size_t>(row0 + i) * Hk + kh) * max_chunks + c) * (Dh + 2); };
+  auto result = [&](int i) {   // where row i of this warp goes
+    const int g = row0 + i;
+    return reinterpret_cast<float4*>(att + static_cast<size_t>(g / group) * H * Dh + static_cast<size_t>(kh * group + g % group) * Dh) + lane;
+  };
   const bool mine = row0 < rows;
   uint4 kreg[VPT], vreg[VPT];
   if (c0 < c1) fetch(kc, c0, kreg);
@@ -651,9 +706,10 @@ __global__ void __launch_bounds__(kAttnThreads, 2)
     place(kreg);
     fetch(vc, c, vreg);
     __syncthreads();
-    const int p0 = lo + c * kAttnChunk;
-    float s[RW][2];
+    const int p0 = c * kAttnChunk;
+    float mx[RW], sum[RW];
     if (mine) {
+      float s[RW][2];
 #pragma unroll
       for (int i = 0; i < RW; ++i) s[i][0] = s[i][1] = 0.f;
       const uint32_t* ka = kv + lane * kRowsStride;
@@ -691,76 +747,69 @@ __global__ void __launch_bounds__(kAttnThreads, 2)
       }
 #pragma unroll
       for (int i = 0; i < RW; ++i) {
-        const bool va = p0 + lane >= first[i] && p0 + lane <= last[i], vb = p0 + lane + 32 >= first[i] && p0 + lane + 32 <= last[i];
-        const float sa = va ? s[i][0] * scale : -INFINITY, sb = vb ? s[i][1] * scale : -INFINITY;
-        float top = fmaxf(mx[i], fmaxf(sa, sb));
-        for (int o = 16; o; o >>= 1) top = fmaxf(top, __shfl_xor_sync(0xffffffffu, top, o));
-        const float ea = va ? __expf(sa - top) : 0.f, eb = vb ? __expf(sb - top) : 0.f;
-        const float keep = sum[i] == 0.f ? 0.f : __expf(mx[i] - top);   // nothing so far: its maximum is -inf, and so may the new one be
+        const float sa = p0 + lane <= last[i] ? s[i][0] * scale : -INFINITY, sb = p0 + lane + 32 <= last[i] ? s[i][1] * scale : -INFINITY;
+        mx[i] = fmaxf(sa, sb);
+        for (int o = 16; o; o >>= 1) mx[i] = fmaxf(mx[i], __shfl_xor_sync(0xffffffffu, mx[i], o));
+        const float ea = __expf(sa - mx[i]), eb = __expf(sb - mx[i]);   // exp(-inf) = 0 for the positions past the row's last
         ps[warp * RW + i][lane] = ea;
         ps[warp * RW + i][lane + 32] = eb;
-        float es = ea + eb;
-        for (int o = 16; o; o >>= 1) es += __shfl_xor_sync(0xffffffffu, es, o);
-        sum[i] = sum[i] * keep + es;
-        mx[i] = top;
-#pragma unroll
-        for (int d = 0; d < 4; ++d) out[i][d] *= keep;
+        sum[i] = ea + eb;
+        for (int o = 16; o; o >>= 1) sum[i] += __shfl_xor_sync(0xffffffffu, sum[i], o);
       }
     }
     __syncthreads();   // the keys have been read
     place(vreg);
     if (c + 1 < c1) fetch(kc, c + 1, kreg);
     __syncthreads();
-    if (mine && lane * 4 < Dh) {
-      const uint32_t* vcol = kv + lane * 2;
-      const int n = min(kAttnChunk, hi - p0);
+    if (mine) {
+      float out[RW][4];
+#pragma unroll
+      for (int i = 0; i < RW; ++i)
+#pragma unroll
+        for (int d = 0; d < 4; ++d) out[i][d] = 0.f;
+      if (lane * 4 < Dh) {
+        const uint32_t* vcol = kv + lane * 2;
+        const int n = min(kAttnChunk, hi - p0);
 #pragma unroll 2
-      for (int p = 0; p < n; p += 4) {
-        float4 w[RW];
+        for (int p = 0; p < n; p += 4) {
+          float4 w[RW];
 #pragma unroll
-        for (int i = 0; i < RW; ++i) w[i] = *reinterpret_cast<const float4*>(&ps[warp * RW + i][p]);
-        // positions that only some rows see are not multiplied into the others: a weight of zero would not hide an infinity
-        const bool every = p0 + p >= all_first && p0 + p + 3 <= all_last;
+          for (int i = 0; i < RW; ++i) w[i] = *reinterpret_cast<const float4*>(&ps[warp * RW + i][p]);
+          // positions that only some rows see are not multiplied into the others: a weight of zero would not hide an infinity
+          const bool every = p0 + p + 3 <= all_last;
 #pragma unroll
-        for (int k = 0; k < 4; ++k) {
-          const uint2 v = *reinterpret_cast<const uint2*>(vcol + (p + k) * kRowsStride);
-          const float2 x = __half22float2(*reinterpret_cast<const __half2*>(&v.x)), y = __half22float2(*reinterpret_cast<const __half2*>(&v.y));
+          for (int k = 0; k < 4; ++k) {
+            const uint2 v = *reinterpret_cast<const uint2*>(vcol + (p + k) * kRowsStride);
+            const float2 x = __half22float2(*reinterpret_cast<const __half2*>(&v.x)), y = __half22float2(*reinterpret_cast<const __half2*>(&v.y));
 #pragma unroll
-          for (int i = 0; i < RW; ++i) {
-            const float wk = k == 0 ? w[i].x : k == 1 ? w[i].y : k == 2 ? w[i].z : w[i].w;
-            if (every || (p0 + p + k >= first[i] && p0 + p + k <= last[i])) {   // the same for the whole warp
-              out[i][0] = fmaf(wk, x.x, out[i][0]);
-              out[i][1] = fmaf(wk, x.y, out[i][1]);
-              out[i][2] = fmaf(wk, y.x, out[i][2]);
-              out[i][3] = fmaf(wk, y.y, out[i][3]);
+            for (int i = 0; i < RW; ++i) {
+              const float wk = k == 0 ? w[i].x : k == 1 ? w[i].y : k == 2 ? w[i].z : w[i].w;
+              if (every || p0 + p + k <= last[i]) {   // the same for the whole warp
+                out[i][0] = fmaf(wk, x.x, out[i][0]);
+                out[i][1] = fmaf(wk, x.y, out[i][1]);
+                out[i][2] = fmaf(wk, y.x, out[i][2]);
+                out[i][3] = fmaf(wk, y.y, out[i][3]);
+              }
             }
           }
         }
       }
-    }
-  }
-  auto result = [&](int i) {   // where row i of this warp goes
-    const int g = row0 + i;
-    return reinterpret_cast<float4*>(att + static_cast<size_t>(g / group) * H * Dh + static_cast<size_t>(kh * group + g % group) * Dh) + lane;
-  };
-  if (spans == 1) {
 #pragma unroll
-    for (int i = 0; i < RW; ++i)
-      if (row0 + i < rows && lane * 4 < Dh)
-        *result(i) = make_float4(out[i][0] / sum[i], out[i][1] / sum[i], out[i][2] / sum[i], out[i][3] / sum[i]);
-    return;
-  }
-  auto span_of = [&](int i, int z) { return part + ((static_cast<size_t>(row0 + i) * Hk + kh) * max_chunks + z) * (Dh + 2); };
-#pragma unroll
-  for (int i = 0; i < RW; ++i)
-    if (row0 + i < rows) {
-      float2* p = reinterpret_cast<float2*>(span_of(i, blockIdx.z));
-      if (lane == 0) p[0] = make_float2(mx[i], sum[i]);
-      if (lane * 4 < Dh) {
-        p[1 + 2 * lane] = make_float2(out[i][0], out[i][1]);
-        p[2 + 2 * lane] = make_float2(out[i][2], out[i][3]);
+      for (int i = 0; i < RW; ++i) {
+        if (p0 > last[i]) continue;   // row i sees nothing of this chunk: its merge stops before
+        if (total == 1) {             // the only chunk of the tile
+          if (lane * 4 < Dh) *result(i) = make_float4(out[i][0] / sum[i], out[i][1] / sum[i], out[i][2] / sum[i], out[i][3] / sum[i]);
+          continue;
+        }
+        float2* p = reinterpret_cast<float2*>(chunk_of(i, c));
+        if (lane == 0) p[0] = make_float2(mx[i], sum[i]);
+        if (lane * 4 < Dh) {
+          p[1 + 2 * lane] = make_float2(out[i][0], out[i][1]);
+          p[2 + 2 * lane] = make_float2(out[i][2], out[i][3]);
+        }
       }
     }
+  }
   __threadfence();
   __syncthreads();
   if (threadIdx.x == 0) {
@@ -770,43 +819,16 @@ __global__ void __launch_bounds__(kAttnThreads, 2)
     if (s_last) *cnt = 0u;   // ready for the next pass
   }
   __syncthreads();
-  if (!s_last) return;
+  if (!s_last || total == 1 || !mine) return;
   __threadfence();
-#pragma unroll 1
-  for (int i = 0; i < RW; ++i) {
-    if (row0 + i >= rows) break;
-    float2 ms = make_float2(-INFINITY, 0.f);
-    if (lane < spans) ms = __ldcg(reinterpret_cast<const float2*>(span_of(i, lane)));
-    float top = ms.x;
-    for (int o = 16; o; o >>= 1) top = fmaxf(top, __shfl_xor_sync(0xffffffffu, top, o));
-    const float w = ms.y == 0.f ? 0.f : __expf(ms.x - top);   // a span that saw no position weighs nothing
-    float tot = ms.y * w;
-    for (int o = 16; o; o >>= 1) tot += __shfl_xor_sync(0xffffffffu, tot, o);
-    float4 acc = make_float4(0.f, 0.f, 0.f, 0.f);
-    for (int z0 = 0; z0 < spans; z0 += 8) {
-      float2 x[8], y[8];
+  int n[RW];
+  float4 res[RW];
 #pragma unroll
-      for (int u = 0; u < 8; ++u) {
-        x[u] = y[u] = make_float2(0.f, 0.f);
-        if (z0 + u < spans && lane * 4 < Dh) {
-          const float2* p = reinterpret_cast<const float2*>(span_of(i, z0 + u));
-          x[u] = __ldcg(p + 1 + 2 * lane);
-          y[u] = __ldcg(p + 2 + 2 * lane);
-        }
-      }
+  for (int i = 0; i < RW; ++i) n[i] = row0 + i < rows ? last[i] / kAttnChunk + 1 : 0;
+  merge_chunks<RW, false>(chunk_of(0, 0), static_cast<size_t>(Hk) * max_chunks * (Dh + 2), n, Dh, lane, res);
 #pragma unroll
-      for (int u = 0; u < 8; ++u) {   // in span order
-        const float wz = __shfl_sync(0xffffffffu, w, (z0 + u) & 31);
-        if (z0 + u < spans) {
-          acc.x = fmaf(wz, x[u].x, acc.x);
-          acc.y = fmaf(wz, x[u].y, acc.y);
-          acc.z = fmaf(wz, y[u].x, acc.z);
-          acc.w = fmaf(wz, y[u].y, acc.w);
-        }
-      }
-    }
-    if (lane * 4 < Dh) *result(i) = make_float4(acc.x / tot, acc.y / tot, acc.z / tot, acc.w / tot);
-  }
+  for (int i = 0; i < RW; ++i)
+    if (row0 + i < rows && lane * 4 < Dh) *result(i) = res[i];
 }
 
 // Greedy decoding on the device: the id of the largest logit (the lowest id among equals, like a host arg-max) becomes
@@ -1105,7 +1127,8 @@ static int nccl_check(int r, const char* what) {
 }
 
 // The device work of one pass over m <= max_batch tokens (ids and position already in R->h_ids): everything is
-// enqueued on `st`, nothing here depends on host-side values that change from pass to pass except `nchunks`.
+// enqueued on `st`, nothing here depends on host-side values that change from pass to pass except `nchunks` and `cut` (the
+// window leaves positions out for some token of the pass).
 static PeerView peer_view(const Runtime* R) {
   PeerView P;
   for (int p = 0; p < kPeerMaxRanks; ++p) {
@@ -1149,7 +1172,7 @@ static int norm_residual(Model* M, Runtime* R, int m, const float* res, bool res
 
 // greedy: the token and the position are already on the device (written by the previous pass's k_argmax_next), and
 // the pass ends with that kernel.
-static int enqueue_pass(Model* M, Runtime* R, int m, bool all_logits, int nchunks, cudaStream_t st, bool greedy = false) {
+static int enqueue_pass(Model* M, Runtime* R, int m, bool all_logits, int nchunks, bool cut, cudaStream_t st, bool greedy = false) {
   cudaError_t e = cudaSuccess;
   if (!greedy) e = cudaMemcpyAsync(R->ids, R->h_ids, (R->max_batch + 1) * sizeof(int), cudaMemcpyHostToDevice, st);
   if (e != cudaSuccess) return cuda_fail("ids upload", e);
@@ -1181,22 +1204,18 @@ static int enqueue_pass(Model* M, Runtime* R, int m, bool all_logits, int nchunk
                                                           R->Tmax);
     {
       const int group = R->H / R->Hk;
-      if (m > 1) {   // tiles of 8, 16 or 32 query rows per kv head
+      if (m > 1 && !cut && debug_knobs().attn_rows) {   // tiles of 8, 16 or 32 query rows per kv head
         const int rows = m * group, rw = rows > 16 ? 4 : rows > 8 ? 2 : 1, tiles = (rows + 8 * rw - 1) / (8 * rw);
-        const int want = std::min({nchunks, kRowsMaxSpans, (2 * sm_count() + R->Hk * tiles - 1) / (R->Hk * tiles)});
+        const int want = std::min(nchunks, (2 * sm_count() + R->Hk * tiles - 1) / (R->Hk * tiles));
         const int per = (nchunks + want - 1) / want, spans = (nchunks + per - 1) / per;
         launch_dep(rw == 4 ? k_attn_rows<4> : rw == 2 ? k_attn_rows<2> : k_attn_rows<1>, dim3(R->Hk, tiles, spans), dim3(kAttnThreads), st,
-                   R->qkv, kc, vc, R->attn_part, R->att, R->attn_done, posp, m, R->H, R->Hk, R->Dh, R->Tmax, R->attn_scale, R->window,
+                   R->qkv, kc, vc, R->attn_part, R->att, R->attn_done, posp, m, R->H, R->Hk, R->Dh, R->Tmax, R->attn_scale, R->max_chunks);
+      } else {
+        const int gh = group % 4 == 0 ? 4 : group % 2 == 0 ? 2 : 1;
+        launch_dep(gh == 4 ? k_attn<4> : gh == 2 ? k_attn<2> : k_attn<1>, dim3(R->H / gh, m, nchunks), dim3(kAttnThreads), st,
+                   R->qkv, kc, vc, R->attn_part, R->att, R->attn_done, posp, R->H, R->Hk, R->Dh, R->Tmax, R->attn_scale, R->window,
                    R->max_chunks);
-      } else if (group % 4 == 0)
-        launch_dep(k_attn<4>, dim3(R->H / 4, 1, nchunks), dim3(kAttnThreads), st, R->qkv, kc, vc, R->attn_part, R->att, R->attn_done,
-                   posp, R->H, R->Hk, R->Dh, R->Tmax, R->attn_scale, R->window, R->max_chunks);
-      else if (group % 2 == 0)
-        launch_dep(k_attn<2>, dim3(R->H / 2, 1, nchunks), dim3(kAttnThreads), st, R->qkv, kc, vc, R->attn_part, R->att, R->attn_done,
-                   posp, R->H, R->Hk, R->Dh, R->Tmax, R->attn_scale, R->window, R->max_chunks);
-      else
-        launch_dep(k_attn<1>, dim3(R->H, 1, nchunks), dim3(kAttnThreads), st, R->qkv, kc, vc, R->attn_part, R->att, R->attn_done,
-                   posp, R->H, R->Hk, R->Dh, R->Tmax, R->attn_scale, R->window, R->max_chunks);
+      }
     }
     if ((rc = linear_device(M, M->mats[R->m_o[l]], R->att, false, m, R->o, R->D, st))) return rc;
     if ((rc = norm_residual(M, R, m, R->o, true, R->ln2[l], st, "all-reduce (o)"))) return rc;
@@ -1291,12 +1310,13 @@ static int forward_chunk(Model* M, Runtime* R, const int* ids_host, int m, bool 
   }
   const int span = R->window > 0 ? std::min(R->window, R->pos + m) : R->pos + m;
   const int nchunks = (span + kAttnChunk - 1) / kAttnChunk;
-  const long long key = (static_cast<long long>(nchunks) << 8) | (m << 1) | (all_logits ? 1 : 0) | (greedy ? 1LL << 62 : 0);
+  const bool cut = R->window > 0 && R->pos + m > R->window;
+  const long long key = (static_cast<long long>(nchunks) << 8) | (m << 1) | (all_logits ? 1 : 0) | (greedy ? 1LL << 62 : 0) | (cut ? 1LL << 61 : 0);
   int rc = kOk;
   auto it = R->graph_exec.find(key);
   if (R->time_collectives && !greedy) {
     // one pass launched directly, with events around every collective; the time between each pair is added up
-    rc = enqueue_pass(M, R, m, all_logits, nchunks, st);
+    rc = enqueue_pass(M, R, m, all_logits, nchunks, cut, st);
     cudaStreamSynchronize(st);
     R->collective_us = 0.0;
     R->collective_calls = static_cast<int>(R->coll_events.size() / 2);
@@ -1316,7 +1336,7 @@ static int forward_chunk(Model* M, Runtime* R, const int* ids_host, int m, bool 
     cudaGraphExec_t exec = nullptr;
     cudaError_t e = cudaStreamBeginCapture(st, cudaStreamCaptureModeRelaxed);
     if (e != cudaSuccess) return cuda_fail("cudaStreamBeginCapture", e);
-    rc = enqueue_pass(M, R, m, all_logits, nchunks, st, greedy);
+    rc = enqueue_pass(M, R, m, all_logits, nchunks, cut, st, greedy);
     e = cudaStreamEndCapture(st, &graph);
     if (rc == kOk && e == cudaSuccess && cudaGraphInstantiate(&exec, graph, 0) == cudaSuccess) {
       R->graph_exec[key] = exec;
@@ -1328,11 +1348,11 @@ static int forward_chunk(Model* M, Runtime* R, const int* ids_host, int m, bool 
       // capture is not possible here (for instance a collective that cannot be captured): run directly from now on
       cudaGetLastError();
       R->graphs = false;
-      rc = enqueue_pass(M, R, m, all_logits, nchunks, st, greedy);
+      rc = enqueue_pass(M, R, m, all_logits, nchunks, cut, st, greedy);
     }
     if (graph) cudaGraphDestroy(graph);
   } else {
-    rc = enqueue_pass(M, R, m, all_logits, nchunks, st, greedy);
+    rc = enqueue_pass(M, R, m, all_logits, nchunks, cut, st, greedy);
   }
   if (rc) return rc;
   R->pos += m;
