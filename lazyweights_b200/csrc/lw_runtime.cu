@@ -1311,7 +1311,8 @@ static int forward_chunk(Model* M, Runtime* R, const int* ids_host, int m, bool 
   const int span = R->window > 0 ? std::min(R->window, R->pos + m) : R->pos + m;
   const int nchunks = (span + kAttnChunk - 1) / kAttnChunk;
   const bool cut = R->window > 0 && R->pos + m > R->window;
-  const long long key = (static_cast<long long>(nchunks) << 8) | (m << 1) | (all_logits ? 1 : 0) | (greedy ? 1LL << 62 : 0) | (cut ? 1LL << 61 : 0);
+  const long long key = (static_cast<long long>(nchunks) << 32) | (static_cast<long long>(m) << 1) | (all_logits ? 1 : 0) |
+                        (greedy ? 1LL << 62 : 0) | (cut ? 1LL << 61 : 0);
   int rc = kOk;
   auto it = R->graph_exec.find(key);
   if (R->time_collectives && !greedy) {

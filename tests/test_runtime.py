@@ -156,3 +156,19 @@ def test_bundle_built_from_a_gguf_runs(tmp_path):
         got = b.forward(ids, all_logits=True)
         assert helpers.rel_err(got, ref) <= 5e-3
         assert b.kernel_error() == 0
+
+
+def test_long_passes_do_not_meet_the_graphs_of_short_ones(tmp_path):
+    """Passes of up to eight tokens are captured and replayed by their shape; a pass of 130 tokens is none of them (its
+    number of tokens once ran into the field beside it and found the graph of two tokens at the same context)."""
+    helpers.build_library()
+    import lazyweights_b200 as lw
+    from lazyweights_b200 import modelgen
+    modelgen.write_model(str(tmp_path / "m"), SHAPE, "Q4_K", "Q4_K", seed=3)
+    ids = np.random.default_rng(8).integers(0, SHAPE["vocab"], 140).astype(np.int32)
+    with lw.Bundle(str(tmp_path / "m"), max_ctx=256, max_batch=136) as b:
+        want = b.forward(ids[:130])
+        for i in range(130, 140, 2):                   # two tokens at 129..192 positions: captured the second time
+            b.forward(ids[i:i + 2])
+        b.reset()
+        assert np.array_equal(b.forward(ids[:130]), want)
