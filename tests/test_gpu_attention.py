@@ -66,11 +66,12 @@ def test_tiles_and_single_tokens_agree_bit_for_bit(tmp_path, heads, kv_heads, he
 
 def test_tokens_of_a_pass_do_not_change_a_query(tmp_path):
     """Passes of two to eight tokens: the products of these row counts are the same arithmetic per row, and attention does
-    not depend on the other tokens of the pass, so neither do the logits."""
+    not depend on the other tokens of the pass, so neither do the logits.  Eight query heads per kv head: the pass of eight
+    tokens has two tiles of rows, the others one, with other spans of chunks from 640 positions on."""
     helpers.build_library()
     import lazyweights_b200 as lw
     ids = np.random.default_rng(5).integers(0, 256, 840).astype(np.int32)
-    with lw.Bundle(_model(tmp_path, 32, 32, 64), max_ctx=1024, max_batch=8) as b:
+    with lw.Bundle(_model(tmp_path, 128, 16, 32), max_ctx=1024, max_batch=8) as b:
         runs = []
         for m in (2, 3, 5, 8):
             b.reset()
