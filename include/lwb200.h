@@ -296,8 +296,9 @@ long long lw_launch_count(void);
 
 /* Test switches (no reference counterpart).  Keys: "max_units" (2..1024: units a block is dealt per launch; smaller
  * values make a product run as several launches over ranges of tile rows, the path very tall matrices take),
- * "wait_limit" (polls after which a device-side wait gives up), "drop_unit" (block 0's producers never copy this unit
- * of their list, so the waits for it run out; -1 = none), "t5_min_rows" (1..65: products of at least this many rows,
+ * "wait_limit" (polls after which a device-side wait gives up), "drop_unit" (block 0 of the one-row kernel never copies this unit
+ * of its list, block 0 of the GEMM over decoded weights this 64-column slab of its first tile, so the waits for it run
+ * out; -1 = none), "t5_min_rows" (1..65: products of at least this many rows,
  * and at most 64, take the decode + tcgen05 kernel; 9 in production), "pairs" (0 / 1: product kernels read the bundle's own code even
  * where a matrix has a pair layout), "attn_rows" (0: passes of several tokens take the attention kernel with a block per token, not
  * the tiled one; passes captured before keep theirs), "reset" (all back to the production values). */

@@ -57,6 +57,7 @@ int launch_gemm_w16(const __half* X, const __half* W, float* Y, int m, int rows,
   a.unscale = a.splits > 1 ? nullptr : unscale;
   a.err = error_word();
   a.wait_limit = debug_knobs().wait_limit;
+  a.drop_slab = debug_knobs().drop_unit;
   a.m = m;
   a.rows = rows;
   a.K = K;

@@ -15,7 +15,9 @@
 //  * A lane of the epilogue holds a weight row, i.e. one output column: a warp's store of one token is 128 bytes.
 //  * Few tiles: K is split (a work item is tile x K range) and each range writes a plane of partial sums,
 //    added in order by k_sum_partials.
-//  * Every wait is bounded; a warp that gives up sets the error word and a block-wide flag that ends every loop.
+//  * Every wait is bounded; a warp that gives up sets the error word and a block-wide flag that ends every loop.  Whoever
+//    gave up, the block ends only after the copies it started have landed and the multiplications it issued are done (waits
+//    with a limit of their own; after a pass that ran through they return at once).
 #pragma once
 #include "lw_tcgen05.cuh"
 
@@ -39,12 +41,13 @@ struct GemmW16Args {
   int slabs;             // 64-column slabs per split (K / 64 / splits)
   int stages;
   int blocks_m;          // 128-row blocks of a tile: 1 or 2
+  int drop_slab;         // a test's lost copy: block 0 never loads this slab of its first item (-1: none)
 };
 
 __global__ void __launch_bounds__(kW16Threads, 1)
     k_gemm_w16(const __grid_constant__ CUtensorMap WM, const __grid_constant__ CUtensorMap XM, const __grid_constant__ GemmW16Args A) {
   extern __shared__ __align__(1024) uint8_t smem_raw[];
-  __shared__ __align__(8) uint64_t full[kW16MaxStages], empty[kW16MaxStages], d_full[2], d_empty[2];
+  __shared__ __align__(8) uint64_t full[kW16MaxStages], empty[kW16MaxStages], d_full[2], d_empty[2], mma_done;
   __shared__ uint32_t tmem_slot[1];
   __shared__ int abort_word;
   volatile int* abort_flag = &abort_word;
@@ -60,6 +63,7 @@ __global__ void __launch_bounds__(kW16Threads, 1)
       mbar_init(smem_addr(d_full + i), 1);
       mbar_init(smem_addr(d_empty + i), 4);
     }
+    mbar_init(smem_addr(&mma_done), 1);
     abort_word = 0;
   }
   if (warp == 1) tmem_alloc(tmem_slot, 512);
@@ -82,20 +86,21 @@ __global__ void __launch_bounds__(kW16Threads, 1)
         for (int k = 0; k < A.slabs; ++k) {
           if (!(ok = t5_wait(empty + s, ph ^ 1u, A.wait_limit, A.err, abort_flag))) break;
           const uint32_t dst = base + s * stage_bytes;
-          mbar_expect(full + s, stage_bytes);
-          for (int i = 0; i < A.blocks_m; ++i)   // rows past the end arrive as zeros
-            tma_load_2d(dst + i * kW16ABytes, &WM, (z * A.slabs + k) * kW16SlabK, (rt * A.blocks_m + i) * kW16Rows, full + s);
-          tma_load_2d(dst + a_bytes, &XM, (z * A.slabs + k) * kW16SlabK, tt * A.ntok, full + s);
+          if (k != A.drop_slab || it != 0) {
+            mbar_expect(full + s, stage_bytes);
+            for (int i = 0; i < A.blocks_m; ++i)   // rows past the end arrive as zeros
+              tma_load_2d(dst + i * kW16ABytes, &WM, (z * A.slabs + k) * kW16SlabK, (rt * A.blocks_m + i) * kW16Rows, full + s);
+            tma_load_2d(dst + a_bytes, &XM, (z * A.slabs + k) * kW16SlabK, tt * A.ntok, full + s);
+          }
           if (++s == A.stages) {
             s = 0;
             ph ^= 1u;
           }
         }
       }
-      // after a wait gave up: the copies still in flight land before the block gives its shared memory back (stages
-      // below s were last filled in round ph, the others in the round before)
-      if (!ok)
-        for (int i = 0; i < A.stages; ++i) mbar_wait(smem_addr(full + i), i < s ? ph : ph ^ 1u, A.err, 1u << 16);
+      // the copies still in flight land before the block gives its shared memory back (stages below s were last filled in
+      // round ph, the others in the round before)
+      for (int i = 0; i < A.stages; ++i) mbar_wait(smem_addr(full + i), i < s ? ph : ph ^ 1u, A.err, 1u << 16);
     }
     __syncwarp();
   } else if (warp == 1) {
@@ -126,6 +131,8 @@ __global__ void __launch_bounds__(kW16Threads, 1)
         }
         if (ok) mma_commit(d_full + db);
       }
+      mma_commit(&mma_done);   // they read shared memory and write tensor memory, which the block is about to give back
+      mbar_wait(smem_addr(&mma_done), 0, A.err, 1u << 16);
     }
     __syncwarp();
   } else {   // ---- epilogue: warp w reads tensor-memory lanes 32 (w % 4) ..

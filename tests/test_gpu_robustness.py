@@ -80,6 +80,28 @@ def test_lost_copy_ends_the_kernel_and_next_product_is_right(lw, ty, n, k):
         assert L.lw_kernel_error() == 0
 
 
+@pytest.mark.parametrize("m,n,k", [(80, 512, 1024), (300, 256, 256), (128, 8192, 512)])
+def test_lost_slab_ends_the_gemm_and_next_product_is_right(lw, m, n, k):
+    """The GEMM over decoded weights: a slab that block 0 never loads.  The wait for it runs out, the block lets its other
+    copies and multiplications finish, the kernel returns with the error word set and the next product is correct.
+    The slab is the second of many, of few (fewer than there are stages), and of a block that would have had more tiles."""
+    import torch
+    q, side, sym, w, rng = helpers.seeded_case("Q4_K" if k % 512 == 0 else "Q6_K", n, k, seed=m + n + k)
+    blob, _, _ = lw.bundle.encode_huf8(sym)
+    with lw.CodedMatrix(blob, n, sym.shape[1], "Q4_K" if k % 512 == 0 else "Q6_K", side) as mat:
+        x = torch.from_numpy(rng.standard_normal((m, k)).astype(np.float16)).cuda()
+        want = mat.linear("m", x).clone()
+        L = lw.lib()
+        assert L.lw_debug_set(b"wait_limit", 20000) == 0 and L.lw_debug_set(b"drop_unit", 1) == 0
+        mat.linear("m", x)
+        torch.cuda.synchronize()                                          # the kernel came back by itself
+        assert L.lw_debug_set(b"reset", 0) == 0
+        assert L.lw_kernel_error() == 1
+        for _ in range(2):
+            assert torch.equal(mat.linear("m", x), want)
+        assert L.lw_kernel_error() == 0
+
+
 def test_token_ids_outside_the_embedding_are_refused(lw, tmp_path):
     from lazyweights_b200 import modelgen
     from tests.test_runtime import SHAPE
