@@ -70,7 +70,11 @@ static int check_side(const Matrix& mx, const uint8_t* side, size_t side_nbytes)
 // need no refill check - shared-memory wavefronts and instructions are what bounds the kernels, not DRAM, which reads
 // 5 % more (paired 4-bit codes: 6.44 instead of 6.12 bits per pair).  Ten bits (16 copies) is where the first step of
 // this went; eight would leave 256 paired symbols no shorter words at all.
-constexpr int kRecodeBits = 9;
+// A matrix that also gets a pair layout is re-coded with ten bits, and only where its code has eleven: nearly all its
+// products read the pair layout, and decoding and encoding it once more costs half of its load again (Q6_K 14336 x 4096,
+// whose code has ten bits: 165 instead of 115 ms on 16 cores).  What reads the other layout and would gain is a Q6_K
+// product of 49 to 64 rows, where the pair layout's units do not fit beside the activations: 57 to 59 us instead of 62.
+constexpr int kRecodeBits = 9, kRecodeBitsPairs = 10;
 static bool recode_wanted() {
   const char* e = getenv("LW_RECODE");
   return !(e && e[0] == '0');
@@ -84,16 +88,25 @@ static int prepare_matrix(const Matrix& mx, const uint8_t* blob, size_t nbytes, 
   if ((rc = check_side(mx, side, side_nbytes))) return rc;
   auto tab = std::make_unique<HuffTable>();
   if ((rc = table_from_lut(v.lut(), *tab))) return rc;
-  if (may_recode && recode_wanted() && mx.fmt != kFmtNone && tab->max_len > kRecodeBits) {
+  // Q6_K / Q5_K rows of whole 512-weight tiles also get a pair layout for the products (LW_PAIRS=0: none); it is built
+  // from the decoded codes, which the walk below writes out
+  static const bool pairs_wanted = [] {
+    const char* e = getenv("LW_PAIRS");
+    return !(e && e[0] == '0');
+  }();
+  const int split = default_split(mx.fmt);
+  const bool grouped = mx.fmt != kFmtNone;
+  const bool pairs = pairs_wanted && grouped && pair_layout_of(mx.fmt) != kFmtNone && mx.K % 512 == 0 && side;
+  const int limit = pairs ? kRecodeBitsPairs : kRecodeBits;
+  if (may_recode && recode_wanted() && mx.fmt != kFmtNone && tab->max_len > limit) {
     // validate and decode the bundle's blob, encode the symbols again with the shorter limit, lay that blob out
     std::vector<uint8_t> symbols(static_cast<size_t>(mx.N) * mx.Ks), shorter;
     if ((rc = walk_blob(v, *tab, default_split(mx.fmt), threads, nullptr, nullptr, symbols.data(), nullptr))) return rc;
-    rc = encode_huf8(symbols.data(), mx.N, mx.Ks, shorter, nullptr, kRecodeBits, threads);
+    rc = encode_huf8(symbols.data(), mx.N, mx.Ks, shorter, nullptr, limit, threads);
     symbols = std::vector<uint8_t>();
     if (rc == kOk) return prepare_matrix(mx, shorter.data(), shorter.size(), side, side_nbytes, threads, im, false);
     if (rc != kErrTooLarge) return rc;   // a payload at the format's 2^32-bit limit: the bundle's own code stays
   }
-  const int split = default_split(mx.fmt);
   std::vector<uint32_t> chain_start, lane_end;
   im.fat.resize(kLutSize);
   fat_table(*tab, mx.fmt, im.fat.data());
@@ -103,14 +116,6 @@ static int prepare_matrix(const Matrix& mx, const uint8_t* blob, size_t nbytes, 
   comparator_table(*tab, mx.fmt, im.cmp.data());
   GroupScan scan;
   scan.quad_syms = 4 * sub_syms(mx.fmt);
-  const bool grouped = mx.fmt != kFmtNone && split == default_split(mx.fmt);
-  // Q6_K / Q5_K rows of whole 512-weight tiles also get a pair layout for the one-row product (LW_PAIRS=0: none); it
-  // is built from the decoded codes, which the same walk writes out
-  static const bool pairs_wanted = [] {
-    const char* e = getenv("LW_PAIRS");
-    return !(e && e[0] == '0');
-  }();
-  const bool pairs = pairs_wanted && grouped && pair_layout_of(mx.fmt) != kFmtNone && mx.K % 512 == 0 && side;
   std::vector<uint8_t> codes;
   if (pairs) codes.resize(static_cast<size_t>(mx.N) * mx.Ks);
   if ((rc = walk_blob(v, *tab, split, threads, &chain_start, &lane_end, pairs ? codes.data() : nullptr, grouped ? &scan : nullptr)))

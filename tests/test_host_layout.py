@@ -231,3 +231,27 @@ def test_pair_code_width_follows_the_data():
         got = _replay_pair_chain(lay["words"], int(lay["group_base"][3]), lane, lay["table"], lay["pad"], 11, 64, 3)
         c = q[32 + lane, 128:256].astype(np.int64) - 32
         assert got == ((c[0::2] & 255) | ((c[1::2] & 255) << 8)).tolist()
+
+
+@pytest.mark.parametrize("ty,k,limit", [("Q6_K", 1024, 10), ("Q5_K", 512, 10), ("Q6_K", 768, 9), ("Q5_K", 256, 9), ("Q4_K", 1024, 9)])
+def test_recoding_limit(ty, k, limit):
+    """Words of the loader's code: at most nine bits, but ten where the matrix gets a pair layout as well (its products
+    read that), and a bundle's code that already keeps to ten bits is then left as it is."""
+    helpers.build_library()
+    import lazyweights_b200 as lw
+    n, seen = 256, set()
+    side = orc.synth_side(ty, n, k, np.random.default_rng(0))
+    for spread in (5.0, 3.0, 11.5, 10.0, 2.5):   # longest words of 8 to 11 bits
+        rng, top = np.random.default_rng(1), {"Q6_K": 63, "Q5_K": 31, "Q4_K": 15}[ty]
+        q = np.clip(np.rint(rng.normal((top + 1) / 2, spread * (top + 1) / 64, (n, k))), 0, top).astype(np.uint8)
+        sym = orc.symbols_of(ty, q)
+        blob, _, _ = lw.bundle.encode_huf8(sym)
+        own = np.frombuffer(blob, np.uint16, 2048)
+        lay = lw.bundle.host_layout(blob, n, sym.shape[1], ty, side)
+        longest = int((own >> 8).max())
+        seen.add(longest)
+        if longest <= limit:
+            assert np.array_equal(lay["lut"], own) and lay["max_len"] == longest
+        else:
+            assert lay["max_len"] <= limit and not np.array_equal(lay["lut"], own)
+    assert 11 in seen and (ty == "Q4_K" or 10 in seen)
