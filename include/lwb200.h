@@ -245,7 +245,8 @@ int lw_cpu_decode(const uint8_t* blob, long long blob_bytes, int N, int Ks, int 
 
 /* Host only (no GPU needed): validates a blob and builds the device layout that lw_matrix_create would upload, for
  * inspection and for tests that replay the kernels' bit arithmetic on the CPU.  info[0..7] = column segments per tile
- * row, pad bits per chain, symbols per refill group of the batch-1 kernel (0 = not used), index bits of its table,
+ * row, pad bits per chain, symbols per refill group of the batch-1 kernel (0 = not used), index bits of its table (9: no
+ * unit classes, every group of four is exact),
  * entries of group_base, entries of unit_class, words of scales behind every work unit, longest unit in words.
  * Returns the number of layout words (negative status on error); each array is filled if its capacity suffices
  * (call once with zero capacities to learn the sizes).  `side` may be null for fmt = LW_FMT_NONE.  No reference

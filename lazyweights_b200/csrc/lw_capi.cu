@@ -54,6 +54,11 @@ struct HostImage {
   uint32_t max_unit = 0, max_tile = 0;
 };
 
+// What the kernels read an image with: a code of at most nine bits through the 512-window table in groups of four, whatever
+// the group that the unit classes stand for.
+static int reader_index_bits(const HostImage& im) { return im.short_code ? 9 : im.index_bits; }
+static int reader_group(int group, int index_bits) { return index_bits == 9 ? 4 : group; }
+
 static int check_side(const Matrix& mx, const uint8_t* side, size_t side_nbytes) {
   if (mx.fmt == kFmtNone) return kOk;
   const size_t want = static_cast<size_t>(mx.N) * (mx.K / 256) * side_bytes(mx.fmt);
@@ -122,11 +127,12 @@ static int prepare_matrix(const Matrix& mx, const uint8_t* blob, size_t nbytes, 
     return rc;
   if (pairs && (rc = build_pairs(codes.data(), mx.N, mx.K, mx.fmt, side, threads, im.pair))) return rc;
   codes = std::vector<uint8_t>();
-  // The batch-1 kernel's table: 1024 windows (codes up to 10 bits; units that hold a longer code are decoded symbol
-  // by symbol) or 2048, 16 copies each; and the group size: units where groups of g symbols are not exact fall back
-  // to groups of two.  Estimated cost per symbol: 8.3 instructions + 10 per group; groups of two cost about 22
-  // (measured: more than their instruction count); the larger table leaves a third fewer staging buffers (+ 8 %);
-  // symbol by symbol costs about 30.  LW_GEMV1_G / LW_GEMV1_IDX override.
+  // A code of at most nine bits (what re-coding gives, and some bundles' own codes) is read through 512 windows in 32 copies
+  // in groups of four, exact for any data.  Otherwise the kernels' table is of 1024 windows in 16 copies (codes up to ten
+  // bits; units that hold a longer code are decoded symbol by symbol) or of 2048 in eight, and the group size is chosen:
+  // units where groups of g symbols are not exact fall back to groups of two.  Estimated cost per symbol: 8.3 instructions
+  // + 10 per group; groups of two cost about 22 (measured: more than their instruction count); the larger table leaves a
+  // third fewer staging buffers (+ 8 %); symbol by symbol costs about 30.  LW_GEMV1_G / LW_GEMV1_IDX override both choices.
   int idx_bits = tab->max_len <= 10 ? 10 : 11, group = 0;
   if (grouped) {
     const int gmax = is_paired(mx.fmt) ? 4 : kScanMaxG;
@@ -265,7 +271,7 @@ static int upload_matrix(Matrix& mx, const HostImage& im, const uint8_t* side, s
   mx.dev.side = side_nbytes ? d + off_side : nullptr;
   mx.dev.unit_slow = im.unit_slow.empty() ? nullptr : d + off_slow;
   mx.dev.group = im.unit_slow.empty() ? 0 : im.group;   // of a refill group; the 512-window readers take fours
-  mx.dev.index_bits = im.short_code ? 9 : im.index_bits;
+  mx.dev.index_bits = reader_index_bits(im);
   mx.dev.N = mx.N;
   mx.dev.K = mx.K;
   mx.dev.Ks = mx.Ks;
@@ -689,7 +695,7 @@ int lw_matrix_info(void* handle, int id, int* N, int* K, int* fmt, long long* bl
 int lw_matrix_plan(void* handle, int id, int* group, int* index_bits, double* slow_fraction) {
   Matrix* mx = matrix_by_id(handle, id);
   if (!mx) return kErrGeneric;
-  if (group) *group = mx->dev.group;
+  if (group) *group = reader_group(mx->dev.group, mx->dev.group ? mx->dev.index_bits : 0);
   if (index_bits) *index_bits = mx->dev.group ? mx->dev.index_bits : 0;
   if (slow_fraction) *slow_fraction = mx->slow_fraction;
   return kOk;
@@ -1065,8 +1071,8 @@ long long lw_host_layout(const uint8_t* blob, long long blob_bytes, int N, int K
   if (rc) return rc;
   info[0] = im.split;
   info[1] = im.pad;
-  info[2] = im.unit_slow.empty() ? 0 : im.group;
-  info[3] = im.index_bits;
+  info[2] = im.unit_slow.empty() ? 0 : reader_group(im.group, reader_index_bits(im));
+  info[3] = reader_index_bits(im);
   info[4] = static_cast<int>(im.group_base.size());
   info[5] = static_cast<int>(im.unit_slow.size());
   info[6] = im.unit_slow.empty() ? 0 : unit_side_words(fmt);

@@ -50,18 +50,39 @@ def _replay_chain(words, base, lane, lut, pad, index_bits, nsym, group, cls):
     return out
 
 
+def _replay_reload_chain(words, base, lane, lut, pad, nsym):
+    """The same for the 512-window table (lw_ring.cuh: ReloadChain): 32 copies want the window one bit further up than the
+    chain has pad bits, so reading starts one bit before the chain; every group of four loads three words at the word its
+    position has reached, and nothing but the position is kept between groups."""
+    bp, shift, out = -1, pad + 1, []
+    a = b = off = 0
+    for i in range(nsym):
+        if i % 4 == 0:
+            q = base + 32 * (bp >> 5) + lane           # rounded down: -1 is the word before the chain
+            w0, w1, w2 = (int(words[q + 32 * j]) if q + 32 * j >= 0 else 0xDEADBEEF for j in range(3))
+            a, b, off = _funnel(w0, w1, bp), _funnel(w1, w2, bp), 0
+        assert off < 32
+        e = int(lut[(_funnel(a, b, off) >> shift) & 511])
+        out.append(e & 255)
+        off += e >> 8
+        if i % 4 == 3 or i == nsym - 1:
+            bp += off
+    return out
+
+
 def _tail_block(ty, q, rng, rows, cols):
     tails = {"Q4_K": [0, 1, 2, 14, 15], "IQ4_XS": [0, 1, 2, 14, 15], "Q5_K": [0, 1, 2, 3, 4, 5, 27, 28, 29, 30, 31],
              "Q6_K": list(range(0, 11)) + list(range(54, 64))}[ty]
     q[rows, cols] = rng.choice(tails, q[rows, cols].shape)
 
 
-@pytest.mark.parametrize("ty,n,k", [("Q6_K", 128, 512), ("Q4_K", 64, 1024), ("Q5_K", 64, 512), ("IQ4_XS", 64, 1024)])
+@pytest.mark.parametrize("ty,n,k", [("Q6_K", 128, 512), ("Q4_K", 64, 1024), ("Q5_K", 64, 512), ("IQ4_XS", 64, 1024), ("Q6_K", 64, 256), ("Q5_K", 64, 768)])
 @pytest.mark.parametrize("force", [None, ("max", "10"), ("max", "11"), ("3", "11")])
 @pytest.mark.parametrize("recode", ["1", "0"])
 def test_grouped_decoder_replayed_on_cpu(monkeypatch, ty, n, k, force, recode):
-    """recode 1: the loader's default, the matrix re-coded with words of at most 10 bits where the bundle's code has
-    11-bit words; 0: the bundle's own code (whose long words make symbol-by-symbol units under a 10-bit table)."""
+    """recode 1: the loader's default, the matrix re-coded with words of at most nine bits (ten, and only from eleven, where
+    it also gets a pair layout); 0: the bundle's own code (whose long words make symbol-by-symbol units under a 10-bit
+    table).  Without forced groups and tables a code of nine bits is read through 512 windows."""
     helpers.build_library()
     import lazyweights_b200 as lw
     monkeypatch.setenv("LW_RECODE", recode)
@@ -76,12 +97,14 @@ def test_grouped_decoder_replayed_on_cpu(monkeypatch, ty, n, k, force, recode):
     lay = lw.bundle.host_layout(blob, n, sym.shape[1], ty, side)
     lut = lay["lut"]                                              # the blob's table, or the re-coded layout's
     own = np.frombuffer(blob, np.uint16, 2048)
-    if recode == "0" or (own >> 8).max() <= 10:
+    limit = 10 if ty in ("Q5_K", "Q6_K") and k % 512 == 0 else 9
+    if recode == "0" or (own >> 8).max() <= limit:
         assert np.array_equal(lut, own) and lay["max_len"] == (own >> 8).max()
     else:
-        assert lay["max_len"] <= 10 and (lut >> 8).max() <= 10 and not np.array_equal(lut, own)
+        assert lay["max_len"] <= limit and (lut >> 8).max() <= limit and not np.array_equal(lut, own)
     split, pad, group, ib = lay["split"], lay["pad"], lay["group"], lay["index_bits"]
-    assert group >= 3 and ib in (10, 11) and pad == 6 and split == (2 if ty == "Q5_K" else 4)
+    short = not force and lay["max_len"] <= 9
+    assert group >= 3 and (ib == 9 and group == 4 if short else ib in (10, 11)) and pad == 6 and split == (2 if ty == "Q5_K" else 4)
     if force:
         assert str(ib) == force[1]
     nsym = 256 // split
@@ -95,7 +118,8 @@ def test_grouped_decoder_replayed_on_cpu(monkeypatch, ty, n, k, force, recode):
             for half in range(2):
                 base = int(lay["group_base"][t * G + 2 * seg + half])
                 for lane in range(0, 32, 5 if cls == 0 else 1):          # every lane of the fallback units
-                    got = _replay_chain(lay["words"], base, lane, lut, pad, ib, nsym, group, cls)
+                    got = (_replay_reload_chain(lay["words"], base, lane, lut, pad, nsym) if short else
+                           _replay_chain(lay["words"], base, lane, lut, pad, ib, nsym, group, cls))
                     row = tr * 64 + half * 32 + lane
                     want = sym[row, tc * 256 + seg * nsym: tc * 256 + (seg + 1) * nsym]
                     assert got == want.tolist(), (t, seg, half, lane, cls)
