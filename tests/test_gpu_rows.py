@@ -103,3 +103,21 @@ def test_scratch_reused_back_to_back(lw):
         got = [mat.linear("m", xs[i]) for i in order]
         for i, y in zip(order, got):
             assert torch.equal(y, want[i])
+
+
+# Sizes whose tiles are 256 weight rows: the last one ragged (64 rows, i.e. one of its two blocks of 128 half full and the
+# other empty), K split over several planes and not, one, two and three token tiles
+@pytest.mark.parametrize("ty,n,k,rows,half", [("Q4_K", 4160, 14336, (80, 300), True), ("Q6_K", 9536, 4096, (257, 600), False)])
+def test_gemm_with_tall_tiles(lw, ty, n, k, rows, half):
+    import torch
+    q, side, sym, w, rng = helpers.seeded_case(ty, n, k, seed=n + k)
+    blob, _, _ = lw.bundle.encode_huf8(sym)
+    wt = torch.from_numpy(w).cuda().double()
+    with lw.CodedMatrix(blob, n, sym.shape[1], ty, side) as mat:
+        for m in rows:
+            x = torch.from_numpy(rng.standard_normal((m, k)).astype(np.float16 if half else np.float32)).cuda()
+            y = torch.full((m + 1, n), -7.0, device="cuda")
+            mat.linear("m", x, out=y[:m])
+            assert (y[m] == -7.0).all()
+            ref = x.double() @ wt.T
+            assert ((y[:m] - ref).abs().amax(1) / ref.abs().amax(1)).max() <= TOL, m
