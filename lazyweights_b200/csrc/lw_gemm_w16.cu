@@ -26,7 +26,9 @@ int launch_gemm_w16(const __half* X, const __half* W, float* Y, int m, int rows,
   // what its bytes take at 95 GB/s per SM or its multiply-adds at 1.1 ns per token and 128 rows, whichever is more; filling and
   // draining about 2 us per launch, and per round where the accumulator is not double-buffered (the tile's results leave
   // meanwhile: 12 ns per token and 128 rows).  Planes of a split cost the extra kernel, about 4 us, and their own traffic:
-  // 0.35 us per MB.  (Q4_K 14336 x 4096: 256 rows win from 257 tokens on, 128 rows up to 256 tokens.)
+  // 0.35 us per MB.  Fitted on Q4_K 14336 x 4096, where 256 rows win from 257 tokens on (300: 77 against 87 us)
+  // and 128 rows up to 256 (128: 61 against 66).  It errs by 3 to 7 per cent on 4096 x 14336 at 128 and 200 tokens, where it takes
+  // 256 rows (63.0 and 72.4 us; 128 rows 61.4 and 67.4).
   a.splits = a.blocks_m = 1;
   double best = 0;
   for (int b = 1; b <= 2; ++b)

@@ -250,7 +250,7 @@ __global__ void __launch_bounds__(256) k_align_halves(const __half* src, uint4* 
 // scheduling).  Four consecutive outputs per thread, PARTS threads per four outputs: part p adds terms p, p + PARTS, ...,
 // then the parts are added with shuffles.  What bounds it is the chain of round trips to L2, one per eight terms of a thread:
 // with one part, 64 terms (the down projection of eight tokens, 8 x 3072 outputs) took 20 us, 24 terms 8 us
-// (now about 5 and 4: a 32-layer pass of eight tokens 5.49 -> 4.30 ms; Q6_K 14336 x 4096, eight rows, 49.6 -> 40.5 us).
+// (now about 5 and 4: a 32-layer pass of eight tokens 5.49 -> 4.30 ms; Q6_K 14336 x 4096, eight rows, 49.6 -> 43.4 us).
 // unscale (may be null): factor per output row j, applied to the finished sum.
 template <int PARTS>
 __global__ void __launch_bounds__(128) k_sum_partials(const float* P, float* __restrict__ Y, int m, int N, int ldy, int terms,

@@ -1,6 +1,6 @@
 // The producer / consumer machinery shared by the persistent decode kernels (batch-1 product lw_gemv1.cuh, 2..8-row
 // product lw_gemvm.cuh, decode to weights lw_decw.cuh, decode to codes lw_decc.cuh, many-row tensor-core product
-// lw_gemm_tc5.cuh): the block's list of work units, the ring of staging buffers that producer lanes fill with bulk
+// lw_gemm_t5.cuh): the block's list of work units, the ring of staging buffers that producer lanes fill with bulk
 // copies, the replicated decode table and the grouped chain reader.  One copy of this code, so that an ordering rule
 // learnt once (wait_released below) holds everywhere.
 //
@@ -23,7 +23,7 @@
 namespace lw {
 
 constexpr int kRingLogCopies = 4;        // the layout's pad allows up to 16 copies of the decode table
-// Copies a kernel keeps: 16 of a 1024-window table, 8 of a 2048-window table, 4 of a 4096-window table (pair layouts)
+// Copies a kernel keeps: 32 of a 512-window table, 16 of a 1024-window table, 8 of a 2048-window table, 4 of a 4096-window table (pair layouts)
 // - 64 KB either way.  (Measured on the pair layout of Q6_K, 14336 x 4096: 8 copies of its 4096-window table = 128 KB
 // leave 10 consumer warps, 23.3 instead of 20.1 us per product; so do units of half the size with either table.)  With 16 copies of the
 // large table (128 KB) too few staging buffers fit beside it, and a block is left with 10 consumer warps instead of 28:
@@ -31,7 +31,7 @@ constexpr int kRingLogCopies = 4;        // the layout's pad allows up to 16 cop
 #ifndef LW_LOG_COPIES_11
 #define LW_LOG_COPIES_11 3
 #endif
-// A code of at most nine bits (the loader re-codes every block-format matrix with that limit: prepare_matrix) needs 512
+// A code of at most nine bits (what the loader re-codes matrices without a pair layout to: prepare_matrix) needs 512
 // windows, of which 32 copies fit: every lane has its own copy in its own bank and a lookup is ONE wavefront instead of
 // 2.0 with 16 copies.
 __host__ __device__ constexpr int ring_log_copies(int index_bits) {

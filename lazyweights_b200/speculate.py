@@ -3,8 +3,9 @@
 Mirrors the reference CLI's `spec` mode (kernels/llmrt.cu:3024-3183): the draft is the continuation of the latest
 earlier occurrence of the last `ngram` tokens (:3105-3112); one forward pass verifies [last token] + drafts (at most
 eight tokens, the fused small-M product); the longest prefix on which the draft equals the greedy argmax is accepted and
-the position is rewound to pos0 + 1 + accepted with rt_set_pos (:3144-3159).  The output equals plain greedy decoding
-(up to float ties), because a verify pass reproduces the single-token logits.
+the position is rewound to pos0 + 1 + accepted with rt_set_pos (:3144-3159).  The output equals plain greedy decoding up to near-ties:
+attention gives a query the same result in either pass, but the products of one row and of several rows add their partial
+sums in different orders, so a verify pass reproduces the single-token logits within rounding, not to the last bit.
 """
 import numpy as np
 
